@@ -30,12 +30,12 @@
 // at every plane.
 //
 // Dykstra's full loop is needed only where some pair |q_i - q_j| exceeds 1
-// (a few percent of the voxels); elsewhere its first sweep is the identity.
-// Stage B tests this per voxel and appends the voxels that need the loop to a
-// per-warp ring queue in shared memory that persists across planes; whenever
-// 32 have gathered, each lane runs the loop on one of them and writes the
-// result to global memory itself (nothing reads Xi^{m+1} during the launch).
-// So the common voxels never wait for a partly idle warp.
+// (5 to 15 % of the voxels, gathered at the phase boundaries); elsewhere its
+// first sweep is the identity.  Stage B tests this per voxel; each row warp
+// has a ring queue in shared memory, appends the voxels that need the loop and
+// goes on.  The Dykstra warps run the loop on queued voxels, two per lane, and
+// write the results to global memory themselves (nothing reads Xi^{m+1} during
+// the launch), so the common voxels never wait for a partly idle warp.
 //
 // HBM traffic per voxel and iteration: Xi and V read and written once, u read
 // once (8(K-1)+1 floats: 68 bytes at K = 3); halo rows/slices and the
@@ -46,6 +46,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "geometry.cuh"
 #include "kernels_plain.cuh"
@@ -93,19 +94,20 @@ struct TileShape {
 #endif
     static constexpr int HALO_WARPS = (Q + 31) / 32 + NHALO_OWN;
     static constexpr int PRODUCER_WARP = MAIN_WARPS + HALO_WARPS;
-    // Dykstra warps run the projection loop of queued voxels; row warp r
-    // queues for Dykstra warp r % NW (about 5 % of the voxels need the loop,
-    // 2.5 sweeps on average; a lane runs one voxel at a time, so the loop's
-    // latency is hidden by many lanes: 6 warps measured faster than 2, 3 or 8)
+    // Dykstra warps run the projection loop of queued voxels: warp w serves the
+    // queues of the row warps w, w + NW, ...
 #ifdef POTTS_DYKSTRA_WARPS
     static constexpr int NW = MAIN_WARPS >= 2 * POTTS_DYKSTRA_WARPS ? POTTS_DYKSTRA_WARPS : (MAIN_WARPS >= 2 ? MAIN_WARPS / 2 : 1);
 #else
-    static constexpr int NW = MAIN_WARPS >= 12 ? 6 : (MAIN_WARPS >= 2 ? MAIN_WARPS / 2 : 1);
+    static constexpr int NW = MAIN_WARPS >= 12 ? (HALO_WARPS > 1 ? 5 : 6) : (MAIN_WARPS >= 2 ? MAIN_WARPS / 2 : 1);
 #endif
+    static constexpr int QPW = (MAIN_WARPS + NW - 1) / NW;  // queues per Dykstra warp
     static constexpr int DYKSTRA_WARP = PRODUCER_WARP + 1;  // the first one
     static constexpr int THREADS = MAIN + 32 * HALO_WARPS + 32 + 32 * NW;
-    static constexpr int QSTRIDE = (3 * K + 1) | 1;  // queue entry: q (3K floats) + state offset; odd stride
-    static constexpr int QN = 128;                     // entries of each Dykstra warp's queue (a power of 2)
+    // queue entry: q (3K floats) and the state offset in whole 16-byte words, an odd number of
+    // them (eight lanes' 16-byte accesses to consecutive entries then fall into different banks)
+    static constexpr int QWORDS = ((3 * K + 4) / 4) | 1;
+    static constexpr int QN = 32 * VPT;  // entries of a row warp's queue: one plane of its voxels
     static constexpr int XI_BYTES = C3 * (R + 2) * NX * ES;
     static constexpr int V_BYTES = C1 * (R + 1) * NVT * ES;
     static constexpr int U_BYTES = (R + 1) * NV * 4;
@@ -117,10 +119,9 @@ struct TileShape {
     static constexpr int OFF_U = OFF_V + D * V_SLOT;
     static constexpr int OFF_VB = OFF_U + D * U_SLOT;
     static constexpr int OFF_Q = OFF_VB + D * VB_SLOT;
-    static constexpr int OFF_QSEQ = OFF_Q + al(NW * QN * QSTRIDE * 4);
-    static constexpr int OFF_QCTL = OFF_QSEQ + al(NW * QN * 4);  // per queue: tail, head, finished writers
+    static constexpr int OFF_QCTL = OFF_Q + al(MAIN_WARPS * QN * QWORDS * 16);  // tails, then heads
     static constexpr int MAX_SEGMENT = 64;  // columns per work item
-    static constexpr int OFF_COLS = OFF_QCTL + al(NW * 16);
+    static constexpr int OFF_COLS = OFF_QCTL + al(MAIN_WARPS * 8);
     static constexpr int OFF_BAR = OFF_COLS + al((MAX_SEGMENT + 3) * 16);
     static constexpr int SMEM = OFF_BAR + 3 * D * 8 + 16;  // + abort flag
     static constexpr int SMEM_ALLOC = SMEM + 128;  // room to align the base to 128 bytes
@@ -186,34 +187,19 @@ struct TiledSmem {
     {
         return reinterpret_cast<float *>(base + S::OFF_VB + slot * S::VB_SLOT);
     }
-    // queue w of voxels waiting for the projection loop: entry data, and per
-    // entry the ticket + 1 of the last entry written there
-    __device__ __forceinline__ float *queue_entry(int w, uint32_t ticket) const
+    // entry `ticket` of row warp r's queue of voxels waiting for the projection loop
+    __device__ __forceinline__ float4 *queue_entry(int r, uint32_t ticket) const
     {
-        return reinterpret_cast<float *>(base + S::OFF_Q) + (w * S::QN + (ticket & (S::QN - 1))) * S::QSTRIDE;
+        return reinterpret_cast<float4 *>(base + S::OFF_Q) + (r * S::QN + (ticket & (S::QN - 1))) * S::QWORDS;
     }
-    __device__ __forceinline__ volatile uint32_t *queue_seq(int w, uint32_t ticket) const
+    // tickets published by row warp r (| kQueueDone after its last one), and tickets taken from it
+    __device__ __forceinline__ uint32_t *q_tail(int r) const
     {
-        return reinterpret_cast<volatile uint32_t *>(base + S::OFF_QSEQ) + w * S::QN + (ticket & (S::QN - 1));
+        return reinterpret_cast<uint32_t *>(base + S::OFF_QCTL) + r;
     }
-    // counters of queue w: tickets handed out to writers, tickets taken by
-    // its Dykstra warp, and row warps writing to it that have finished
-    __device__ __forceinline__ uint32_t *q_tail(int w) const
+    __device__ __forceinline__ uint32_t *q_head(int r) const
     {
-        return reinterpret_cast<uint32_t *>(base + S::OFF_QCTL) + 4 * w;
-    }
-    __device__ __forceinline__ volatile uint32_t *q_head(int w) const
-    {
-        return reinterpret_cast<volatile uint32_t *>(base + S::OFF_QCTL) + 4 * w + 1;
-    }
-    __device__ __forceinline__ uint32_t *q_done(int w) const
-    {
-        return reinterpret_cast<uint32_t *>(base + S::OFF_QCTL) + 4 * w + 2;
-    }
-    // row warps that write to queue w
-    __device__ __forceinline__ static uint32_t q_writers(int w)
-    {
-        return (uint32_t)((S::MAIN_WARPS - 1 - w) / S::NW + 1);
+        return reinterpret_cast<uint32_t *>(base + S::OFF_QCTL) + S::MAIN_WARPS + r;
     }
     __device__ __forceinline__ uint64_t *full(int slot) const
     {
@@ -265,9 +251,9 @@ __device__ __forceinline__ void stage_a_chunk(const TiledSmem<K, R, NT, VPT, ST>
         for (int i = 0; i < K - 1; ++i) stv<VPT>(vb + T::v_at(i, rr, off), z);
         return;
     }
-    const bool pr = row > ci.y, hr = row + 1 < ci.z;
+    [[maybe_unused]] const bool pr = row > ci.y, hr = row + 1 < ci.z;
     const bool pc = row_in_col(sm.cols()[p - 1], row);
-    const bool hc = row_in_col(sm.cols()[p + 1], row);
+    [[maybe_unused]] const bool hc = row_in_col(sm.cols()[p + 1], row);
     const ST *xs = sm.xi_slot(sc), *xp = sm.xi_slot(sp);
     const ST *vs = sm.v_slot(sc);
     const float *us = sm.u_slot(sc);
@@ -313,71 +299,43 @@ __device__ __forceinline__ void stage_a_chunk(const TiledSmem<K, R, NT, VPT, ST>
                 obar[i][j + 1] = in1 ? Store<ST>::round(vbar[i].y) : 0.0f;
             }
         }
-    } else if constexpr (VPT == 2) {
-        // both slices with paired FP32 instructions
-        float2 x[S::C3], xin[K - 1], xr[K - 1], xc[K - 1], v[K - 1], vn[K - 1], vbar[K - 1];
-#pragma unroll
-        for (int comp = 0; comp < S::C3; ++comp) x[comp] = Store<ST>::ld2(xs + T::xi_at(comp, rr + 1, off + XH));
-#pragma unroll
-        for (int i = 0; i < K - 1; ++i) {
-            const float2 before = Store<ST>::ld2(xs + T::xi_at(3 * i, rr + 1, off + XH - 2));  // slices nb-2, nb-1
-            xin[i] = f2(before.y, x[3 * i].x);
-            xr[i] = Store<ST>::ld2(xs + T::xi_at(3 * i + 1, rr, off + XH));
-            xc[i] = Store<ST>::ld2(xp + T::xi_at(3 * i + 2, rr + 1, off + XH));
-            v[i] = Store<ST>::ld2(vs + T::vt_at(i, rr, off));
-        }
-        const float2 u2 = reinterpret_cast<const float2 *>(us)[T::v_at(0, rr, off) / 2];
-        const bool second = nb + 1 < tp.ns;
-        const float fr = pr ? 1.0f : 0.0f, gr = hr ? 1.0f : 0.0f, fc = pc ? 1.0f : 0.0f, gc = hc ? 1.0f : 0.0f;
-        const float2 d = primal_pair<K>(vn, vbar, v, x, xin, xr, xc, f2(nb > 0 ? 1.0f : 0.0f, 1.0f),
-                                        f2(second ? 1.0f : 0.0f, nb + 2 < tp.ns ? 1.0f : 0.0f), f2(fr), f2(gr),
-                                        f2(fc), f2(gc), u2, pp.c, pp.lam, pp.tau1);
-        if (store_v) dqmax = fmaxf(dqmax, second ? fmaxf(d.x, d.y) : d.x);
-#pragma unroll
-        for (int i = 0; i < K - 1; ++i) {
-            onew[i][0] = vn[i].x;
-            obar[i][0] = Store<ST>::round(vbar[i].x);  // Vbar as if stored
-            onew[i][1] = second ? vn[i].y : 0.0f;
-            obar[i][1] = second ? Store<ST>::round(vbar[i].y) : 0.0f;
-        }
     } else {
-        float x[S::C3][VPT], xn[K - 1][VPT], xr[K - 1][VPT], xc[K - 1][VPT], v[K - 1][VPT], u[VPT];
+        // exact arithmetic, two slices at a time with paired FP32 instructions
+        float x[S::C3][VPT], xn[K - 1], xr[K - 1][VPT], xc[K - 1][VPT], v[K - 1][VPT], u[VPT];
 #pragma unroll
         for (int comp = 0; comp < S::C3; ++comp) ldv<VPT>(x[comp], xs + T::xi_at(comp, rr + 1, off + XH));
 #pragma unroll
         for (int i = 0; i < K - 1; ++i) {
-            ldv<VPT>(xn[i], xs + T::xi_at(3 * i, rr + 1, off + XH - VPT));  // the chunk before: slices nb-VPT .. nb-1
+            xn[i] = Store<ST>::ld2(xs + T::xi_at(3 * i, rr + 1, off + XH - 2)).y;  // slice nb-1
             ldv<VPT>(xr[i], xs + T::xi_at(3 * i + 1, rr, off + XH));
             ldv<VPT>(xc[i], xp + T::xi_at(3 * i + 2, rr + 1, off + XH));
             ldv<VPT>(v[i], vs + T::vt_at(i, rr, off));
         }
         ldv<VPT>(u, us + T::v_at(0, rr, off));
+        const float fr = pr ? 1.0f : 0.0f, gr = hr ? 1.0f : 0.0f, fc = pc ? 1.0f : 0.0f, gc = hc ? 1.0f : 0.0f;
 #pragma unroll
-        for (int j = 0; j < VPT; ++j) {
-            const int n = nb + j;
-            float xi_j[S::C3], xin_j[K - 1], xir_j[K - 1], xic_j[K - 1], v_j[K - 1], vn[K - 1], vbar[K - 1];
+        for (int j = 0; j < VPT; j += 2) {
+            float2 xj[S::C3], xinj[K - 1], xrj[K - 1], xcj[K - 1], vj[K - 1], vn[K - 1], vbar[K - 1];
 #pragma unroll
-            for (int comp = 0; comp < S::C3; ++comp) xi_j[comp] = x[comp][j];
-#pragma unroll
-            for (int i = 0; i < K - 1; ++i) {
-                xin_j[i] = (j == 0) ? xn[i][VPT - 1] : x[3 * i][j - 1];
-                xir_j[i] = xr[i][j];
-                xic_j[i] = xc[i][j];
-                v_j[i] = v[i][j];
-            }
-            float d = 0.0f;
-            if (n < tp.ns) {
-                d = primal_voxel<K>(vn, vbar, v_j, xi_j, xin_j, xir_j, xic_j, n > 0, n + 1 < tp.ns, pr, hr, pc, hc,
-                                    u[j], pp.c, pp.lam, pp.tau1);
-            } else {
-#pragma unroll
-                for (int i = 0; i < K - 1; ++i) vn[i] = vbar[i] = 0.0f;
-            }
-            if (store_v) dqmax = fmaxf(dqmax, d);
+            for (int comp = 0; comp < S::C3; ++comp) xj[comp] = f2(x[comp][j], x[comp][j + 1]);
 #pragma unroll
             for (int i = 0; i < K - 1; ++i) {
-                onew[i][j] = vn[i];
-                obar[i][j] = Store<ST>::round(vbar[i]);  // Vbar as if stored
+                xinj[i] = f2(j == 0 ? xn[i] : x[3 * i][j - 1], x[3 * i][j]);
+                xrj[i] = f2(xr[i][j], xr[i][j + 1]);
+                xcj[i] = f2(xc[i][j], xc[i][j + 1]);
+                vj[i] = f2(v[i][j], v[i][j + 1]);
+            }
+            const bool in0 = nb + j < tp.ns, in1 = nb + j + 1 < tp.ns;
+            const float2 d = primal_pair<K>(vn, vbar, vj, xj, xinj, xrj, xcj, f2(nb + j > 0 ? 1.0f : 0.0f, 1.0f),
+                                            f2(in1 ? 1.0f : 0.0f, nb + j + 2 < tp.ns ? 1.0f : 0.0f), f2(fr), f2(gr),
+                                            f2(fc), f2(gc), f2(u[j], u[j + 1]), pp.c, pp.lam, pp.tau1);
+            if (store_v) dqmax = fmaxf(dqmax, in0 ? (in1 ? fmaxf(d.x, d.y) : d.x) : 0.0f);
+#pragma unroll
+            for (int i = 0; i < K - 1; ++i) {
+                onew[i][j] = in0 ? vn[i].x : 0.0f;
+                obar[i][j] = in0 ? Store<ST>::round(vbar[i].x) : 0.0f;  // Vbar as if stored
+                onew[i][j + 1] = in1 ? vn[i].y : 0.0f;
+                obar[i][j + 1] = in1 ? Store<ST>::round(vbar[i].y) : 0.0f;
             }
         }
     }
@@ -464,111 +422,161 @@ __device__ __forceinline__ void stage_a_nhalo(const TiledSmem<K, R, NT, VPT, ST>
     for (int i = 0; i < K - 1; ++i) vb[T::v_at(i, rr, NT)] = Store<ST>::round(vbar[i]);
 }
 
-// The Dykstra warp: runs the projection loop of the voxels that the row warps
-// queue.  It sleeps until kBatch voxels have gathered in its queue (or the
-// row warps are done), then each lane takes one voxel, runs it a sweep at a
-// time and, once it is done, stores the result and takes the next waiting
-// ticket, until the queue is empty and every lane has finished.  It returns
-// when every row warp has finished and the queue is empty, or when the block
-// aborts.  Every wait is bounded.
-constexpr int kQueueSpin = 1 << 20;   // polls of an entry's publication flag
+constexpr uint32_t kQueueDone = 0x80000000u;
+constexpr int kQueueWait = 1 << 22;   // polls (~200 ns each) of a full queue before a row warp gives up
 constexpr int kIdleRounds = 1 << 23;  // idle polls (~400 ns each) while the row warps work
-#ifdef POTTS_DYKSTRA_BATCH
-constexpr uint32_t kBatch = POTTS_DYKSTRA_BATCH;
-#else
-constexpr uint32_t kBatch = 1;  // queued voxels that start a batch (larger batches measured no faster)
-#endif
 
+__device__ __forceinline__ uint32_t ld_acquire_cta(const uint32_t *p)
+{
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_cta(uint32_t *p, uint32_t v)
+{
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
+}
+
+// Slot `j` of a lane's value: a float2 holds two voxels, a float one.
+__device__ __forceinline__ void set_slot(float2 &v, int j, float x) { (j ? v.y : v.x) = x; }
+__device__ __forceinline__ void set_slot(float &v, int, float x) { v = x; }
+__device__ __forceinline__ float get_slot(const float2 &v, int j) { return j ? v.y : v.x; }
+__device__ __forceinline__ float get_slot(const float &v, int) { return v; }
+
+// A Dykstra warp: runs the projection loop of the voxels that its row warps
+// queue.  A lane holds two voxels (one for K > 4, whose corrections fill the
+// registers) and runs sweeps of both with the paired instructions; a voxel that
+// is done is stored, and free slots take the next waiting entries once kRefill
+// of them are free.  A sweep is a serial chain of about a hundred dependent
+// operations, so its latency and the instructions around it (polling, taking,
+// storing), not the arithmetic, set the warp's rate: the two voxels share both,
+// two sweeps share the polling (at K = 4 that loop spilled), and the warp sleeps
+// while fewer than half of its slots hold a voxel and more are to come.  At 512 x
+// 512 x 256, K = 3, 13 % of the voxels in the loop and 4.5 sweeps each (iterations
+// 2 to 40): 1.016 -> 0.799 ms per iteration in the fast arithmetic (one voxel per
+// lane, entries shared through one atomic tail per Dykstra warp, and row warps
+// that ran the loop themselves when the queue was full), of which 0.63 ms are
+// the rest of the kernel, 0.07 ms the queueing and 0.02 ms the second stores; four
+// voxels per lane spilled, more Dykstra warps took issue slots from the row warps
+// (0.84 ms with 6), and row warps that joined in held up their neighbours (1.0 ms).
+// Returns when every row warp has finished and its queues are empty, or when the
+// block aborts.  Every wait is bounded.
 template <int K, int R, int NT, int VPT, typename ST, bool FAST>
 __device__ __forceinline__ void dykstra_worker(const TiledSmem<K, R, NT, VPT, ST> &sm, int w, const TiledParams &tp,
                                                DykstraThresholds thr, ST *__restrict__ Xout, volatile int *abort)
 {
+    using S = TileShape<K, R, NT, VPT, ST>;
     constexpr int kPairs = K * (K - 1) / 2;
+    constexpr int kSlots = K <= 4 ? 2 : 1;
+    constexpr int kAll = 32 * kSlots, kRefill = kAll / 4, kFreeMax = kAll / 2;
+    constexpr int kSweeps = K <= 3 ? 2 : 1;  // between two looks at the queues
+    constexpr int kVec = (3 * K + 4) / 4;    // 16-byte words of an entry in use
+    using F = std::conditional_t<kSlots == 2, float2, float>;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    using T = TiledSmem<K, R, NT, VPT, ST>;
-    volatile uint32_t *tail_v = sm.q_tail(w);
-    volatile uint32_t *done_v = sm.q_done(w);
-    float qe[K][3], P[kPairs][3];
-    int64_t o = 0;
-    int sweeps = 0;
-    bool active = false, batch = false;
-    uint32_t next = 0;  // next ticket to hand out (the same in every lane)
+    // lane k polls the k-th of the warp's queues and keeps its head
+    const int my_queue = w + S::NW * lane;
+    const bool polls = lane < S::QPW && my_queue < S::MAIN_WARPS;
+    uint32_t head = 0;
+    int last = 0;  // the queue taken from last
+    F q[K][3], P[kPairs][3];
+#pragma unroll
+    for (int i = 0; i < K; ++i) q[i][0] = q[i][1] = q[i][2] = F{};
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) P[p][0] = P[p][1] = P[p][2] = F{};
+    uint32_t off[kSlots];
+    int sweeps[kSlots];  // of the voxel in the slot; negative: the slot is free
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) off[j] = 0u, sweeps[j] = -1;
     int idle_rounds = 0;
     while (true) {
-        if (!batch) {
-            // a row warp publishes its last entries before it counts itself
-            // done, so `done` is read before the tail
-            const bool done = __shfl_sync(0xffffffffu, (int)(*done_v == T::q_writers(w)), 0) != 0;
-            const uint32_t avail = __shfl_sync(0xffffffffu, *tail_v, 0) - next;
-            if (avail >= kBatch || (done && avail > 0u)) {
-                batch = true;
-            } else if (done || __shfl_sync(0xffffffffu, *abort, 0)) {
-                break;
-            } else {
-                if (++idle_rounds > kIdleRounds) {
-                    *abort = 1;
-                    break;
-                }
-                __nanosleep(400);
-                continue;
-            }
-            idle_rounds = 0;
-        }
-        const uint32_t avail = __shfl_sync(0xffffffffu, *tail_v, 0) - next;
-        const unsigned idle = __ballot_sync(0xffffffffu, !active);
-        if (avail > 0u && idle != 0u) {
-            const uint32_t take = min((uint32_t)__popc(idle), avail);
-            const uint32_t rank = (uint32_t)__popc(idle & below);
-            if (!active && rank < take) {
-                const uint32_t ticket = next + rank;
-                volatile uint32_t *seq = sm.queue_seq(w, ticket);
-                int spins = 0;
-                bool published = *seq == ticket + 1u;
-                while (!published && spins < kQueueSpin && !*abort) {
-                    ++spins;
-                    published = *seq == ticket + 1u;
-                }
-                if (published) {
-                    __threadfence_block();
-                    const float *ent = sm.queue_entry(w, ticket);
+        unsigned idle[kSlots];
+        int n_free = 0;
 #pragma unroll
-                    for (int i = 0; i < K; ++i) {
-                        qe[i][0] = ent[3 * i];
-                        qe[i][1] = ent[3 * i + 1];
-                        qe[i][2] = ent[3 * i + 2];
+        for (int j = 0; j < kSlots; ++j) {
+            idle[j] = __ballot_sync(0xffffffffu, sweeps[j] < 0);
+            n_free += __popc(idle[j]);
+        }
+        if (n_free >= kRefill) {
+            const uint32_t tail = polls ? ld_acquire_cta(sm.q_tail(my_queue)) : kQueueDone;
+            const uint32_t waiting = polls ? (tail & ~kQueueDone) - head : 0u;
+            const unsigned has = __ballot_sync(0xffffffffu, waiting != 0u);
+            if (has != 0u) {
+                const unsigned after = has & ~((2u << last) - 1u);  // the queues in turn
+                last = __ffs((int)(after ? after : has)) - 1;
+                const uint32_t first = __shfl_sync(0xffffffffu, head, last);
+                const uint32_t take = min((uint32_t)n_free, __shfl_sync(0xffffffffu, waiting, last));
+                const int queue = w + S::NW * last;
+                __syncwarp();  // the polling lane's acquire, before the other lanes' reads
+                uint32_t before = 0;
+#pragma unroll
+                for (int j = 0; j < kSlots; ++j) {
+                    const uint32_t rank = before + (uint32_t)__popc(idle[j] & below);
+                    before += (uint32_t)__popc(idle[j]);
+                    if (sweeps[j] < 0 && rank < take) {
+                        const float4 *e = sm.queue_entry(queue, first + rank);
+                        float v[4 * kVec];
+#pragma unroll
+                        for (int k = 0; k < kVec; ++k) {
+                            const float4 t = e[k];
+                            v[4 * k] = t.x, v[4 * k + 1] = t.y, v[4 * k + 2] = t.z, v[4 * k + 3] = t.w;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 3 * K; ++i) set_slot(q[i / 3][i % 3], j, v[i]);
+                        off[j] = __float_as_uint(v[3 * K]);
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p)
+#pragma unroll
+                            for (int a = 0; a < 3; ++a) set_slot(P[p][a], j, 0.0f);
+                        sweeps[j] = 0;
                     }
-                    o = (int64_t)(uint32_t)__float_as_int(ent[3 * K]);
-#pragma unroll
-                    for (int p = 0; p < kPairs; ++p) P[p][0] = P[p][1] = P[p][2] = 0.0f;
-                    sweeps = 0;
-                    active = true;
+                }
+                __syncwarp();
+                if (lane == last) {
+                    head += take;
+                    st_release_cta(sm.q_head(my_queue), head);  // the taken entries are free again
+                }
+                idle_rounds = 0;
+                n_free -= (int)take;
+                if (n_free > kFreeMax) continue;  // look at the other queues first
+            } else if (n_free > kFreeMax) {
+                if (__all_sync(0xffffffffu, (tail & kQueueDone) != 0u)) {
+                    if (n_free == kAll) break;  // nothing left, nothing to come
                 } else {
-                    *abort = 1;
+                    if (__shfl_sync(0xffffffffu, *abort, 0)) break;
+                    if (++idle_rounds > kIdleRounds) {
+                        *abort = 1;
+                        break;
+                    }
+                    __nanosleep(400);
+                    continue;
                 }
             }
-            next += take;
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0) *sm.q_head(w) = next;  // the taken entries' slots are free again
         }
-        if (!__any_sync(0xffffffffu, active)) {
-            batch = false;  // the queue ran dry: wait for the next batch
-            if (__shfl_sync(0xffffffffu, *abort, 0)) break;
-            continue;
-        }
-        if (active) {
-            bool exit;
-            if constexpr (FAST)
-                exit = fast::dykstra_sweep<K>(qe, P);
-            else
-                exit = dykstra_sweep<K>(qe, P, thr);
-            if (exit || ++sweeps == 20) {
+#pragma unroll 1
+        for (int rep = 0; rep < kSweeps; ++rep) {
+            bool done[kSlots];
+            if constexpr (FAST) {
+                const F step = fast::dykstra_sweep<K, F>(q, P);
 #pragma unroll
-                for (int i = 0; i < K - 1; ++i)
+                for (int j = 0; j < kSlots; ++j) done[j] = get_slot(step, j) < fast::kExit2;
+            } else if constexpr (kSlots == 2) {
+                float2 step;
+                dykstra_sweep_pair<K>(q, P, thr, step);
+                done[0] = step.x < thr.exit_below, done[1] = step.y < thr.exit_below;
+            } else {
+                done[0] = dykstra_sweep<K>(q, P, thr);
+            }
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) Xout[(3 * i + a) * tp.plane_w + o] = Store<ST>::st(qe[i][a]);
-                active = false;
+            for (int j = 0; j < kSlots; ++j) {
+                if (sweeps[j] >= 0 && (++sweeps[j] == 20 || done[j])) {
+                    ST *x = Xout + off[j];
+#pragma unroll
+                    for (int i = 0; i < K - 1; ++i)
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) x[(3 * i + a) * tp.plane_w] = Store<ST>::st(get_slot(q[i][a], j));
+                    sweeps[j] = -1;
+                }
             }
         }
     }
@@ -577,11 +585,11 @@ __device__ __forceinline__ void dykstra_worker(const TiledSmem<K, R, NT, VPT, ST
 // Stage B: dual step at ring position p (slot sc; slot sn holds plane p+1)
 // for VPT slices n0+VPT*q .. of tile row rr.  Called by every lane of the row
 // warps (warp-wide ballots); voxels that need the projection loop go to the
-// block's queue.
+// warp's queue.  False when the block is aborting.
 template <int K, int R, int NT, int VPT, typename ST, bool FAST>
-__device__ __forceinline__ void stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST> &sm, const TiledParams &tp, int p,
+__device__ __forceinline__ bool stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST> &sm, const TiledParams &tp, int p,
                                               int sc, int sn, int r0, int rr, int n0, int q, float tau2,
-                                              DykstraThresholds thr, ST *__restrict__ Xout)
+                                              DykstraThresholds thr, ST *__restrict__ Xout, volatile int *abort)
 {
     using S = TileShape<K, R, NT, VPT, ST>;
     using T = TiledSmem<K, R, NT, VPT, ST>;
@@ -638,28 +646,6 @@ __device__ __forceinline__ void stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST>
                         qv[j + 1][i][a] = q2[i][a].y;
                     }
             }
-        } else if constexpr (VPT == 2) {
-            float2 x[S::C3], b[K - 1], bn[K - 1], br[K - 1], bc[K - 1], q2[K][3];
-#pragma unroll
-            for (int comp = 0; comp < S::C3; ++comp)
-                x[comp] = Store<ST>::ld2(xs + T::xi_at(comp, rr + 1, off + XH));
-#pragma unroll
-            for (int i = 0; i < K - 1; ++i) {
-                b[i] = reinterpret_cast<const float2 *>(vb0)[T::v_at(i, rr, off) / 2];
-                bn[i] = f2(b[i].y, vb0[T::v_at(i, rr, off + 2)]);
-                br[i] = reinterpret_cast<const float2 *>(vb0)[T::v_at(i, rr + 1, off) / 2];
-                bc[i] = reinterpret_cast<const float2 *>(vb1)[T::v_at(i, rr, off) / 2];
-            }
-            dual_build_q_pair<K>(q2, x, b, bn, br, bc, f2(nb + 1 < tp.ns ? 1.0f : 0.0f, nb + 2 < tp.ns ? 1.0f : 0.0f),
-                                 f2(hr ? 1.0f : 0.0f), f2(hc ? 1.0f : 0.0f), tau2);
-            need = dual_needs_loop_pair<K>(q2, thr) & (nb + 1 < tp.ns ? 3u : 1u);
-#pragma unroll
-            for (int i = 0; i < K; ++i)
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    qv[0][i][a] = q2[i][a].x;
-                    qv[1][i][a] = q2[i][a].y;
-                }
         } else {
             float x[S::C3][VPT], b[K - 1][VPT], bnext[K - 1], br[K - 1][VPT], bc[K - 1][VPT];
 #pragma unroll
@@ -671,20 +657,32 @@ __device__ __forceinline__ void stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST>
                 ldv<VPT>(br[i], vb0 + T::v_at(i, rr + 1, off));
                 ldv<VPT>(bc[i], vb1 + T::v_at(i, rr, off));
             }
+            const float2 fr = f2(hr ? 1.0f : 0.0f), fc = f2(hc ? 1.0f : 0.0f);
 #pragma unroll
-            for (int j = 0; j < VPT; ++j) {
-                float xi_j[S::C3], b_j[K - 1], bn_j[K - 1], br_j[K - 1], bc_j[K - 1];
+            for (int j = 0; j < VPT; j += 2) {
+                float2 xj[S::C3], bj[K - 1], bnj[K - 1], brj[K - 1], bcj[K - 1], q2[K][3];
 #pragma unroll
-                for (int comp = 0; comp < S::C3; ++comp) xi_j[comp] = x[comp][j];
+                for (int comp = 0; comp < S::C3; ++comp) xj[comp] = f2(x[comp][j], x[comp][j + 1]);
 #pragma unroll
                 for (int i = 0; i < K - 1; ++i) {
-                    b_j[i] = b[i][j];
-                    bn_j[i] = (j < VPT - 1) ? b[i][j + 1] : bnext[i];
-                    br_j[i] = br[i][j];
-                    bc_j[i] = bc[i][j];
+                    bj[i] = f2(b[i][j], b[i][j + 1]);
+                    bnj[i] = f2(b[i][j + 1], j + 2 < VPT ? b[i][j + 2] : bnext[i]);
+                    brj[i] = f2(br[i][j], br[i][j + 1]);
+                    bcj[i] = f2(bc[i][j], bc[i][j + 1]);
                 }
-                dual_build_q<K>(qv[j], xi_j, b_j, bn_j, br_j, bc_j, nb + j + 1 < tp.ns, hr, hc, tau2);
-                if (nb + j < tp.ns && !dual_first_sweep_is_identity<K>(qv[j], thr)) need |= 1u << j;
+                dual_build_q_pair<K>(q2, xj, bj, bnj, brj, bcj,
+                                     f2(nb + j + 1 < tp.ns ? 1.0f : 0.0f, nb + j + 2 < tp.ns ? 1.0f : 0.0f), fr, fc,
+                                     tau2);
+                need |= (dual_needs_loop_pair<K>(q2, thr) &
+                         ((nb + j < tp.ns ? 1u : 0u) | (nb + j + 1 < tp.ns ? 2u : 0u)))
+                        << j;
+#pragma unroll
+                for (int i = 0; i < K; ++i)
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        qv[j][i][a] = q2[i][a].x;
+                        qv[j + 1][i][a] = q2[i][a].y;
+                    }
             }
         }
     }
@@ -692,8 +690,8 @@ __device__ __forceinline__ void stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST>
     // Every voxel's q is stored at once, whole vectors in every lane (no lane
     // takes a separate path for its loop voxels).  The voxels that need the
     // projection loop are stored again, with the loop's result, by the Dykstra
-    // warp that runs them (their queue entries are published behind a block
-    // fence, after this store) or by the lane itself when the queue is full.
+    // warp that runs them (it takes their entries after the queue's release
+    // below, which follows this store).
     if (live) {
         if (nb + VPT <= tp.ns) {
 #pragma unroll
@@ -717,9 +715,9 @@ __device__ __forceinline__ void stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST>
         }
     }
 
-    // the loop voxels of the whole warp go to the block's queue in one
-    // reservation (the Dykstra warp runs them); when it is full, each lane
-    // runs the loop of its own voxels
+    // the loop voxels of the whole warp go to its queue; the Dykstra warps work
+    // through it far faster than the row warp fills it, so a full queue (which
+    // holds a whole plane of the warp) is waited for
     unsigned bal[VPT];
     uint32_t total = 0;
 #pragma unroll
@@ -727,66 +725,35 @@ __device__ __forceinline__ void stage_b_chunk(const TiledSmem<K, R, NT, VPT, ST>
         bal[j] = __ballot_sync(0xffffffffu, (need >> j) & 1u);
         total += (uint32_t)__popc(bal[j]);
     }
-    if (total == 0u) return;
-    uint32_t base = 0;
-    bool queued = false;
-    const int w = (threadIdx.x >> 5) % S::NW;
-    if (lane == 0) {
-        uint32_t *tail = sm.q_tail(w);
-        uint32_t t = *reinterpret_cast<volatile uint32_t *>(tail);
-        for (int tries = 0; tries < 64; ++tries) {
-            if (t + total - *sm.q_head(w) > (uint32_t)S::QN) break;  // no room
-            const uint32_t prev = atomicCAS(tail, t, t + total);
-            if (prev == t) {
-                queued = true;
-                base = t;
-                break;
-            }
-            t = prev;
-        }
+    if (total == 0u) return true;
+    const int w = threadIdx.x >> 5;
+    uint32_t ticket = *reinterpret_cast<volatile uint32_t *>(sm.q_tail(w));  // only this warp writes it
+    const uint32_t next = ticket + total;
+    for (int tries = 0; __any_sync(0xffffffffu, next - ld_acquire_cta(sm.q_head(w)) > (uint32_t)S::QN); ++tries) {
+        if (tries >= kQueueWait) *abort = 1;
+        if (__any_sync(0xffffffffu, *abort != 0)) return false;
+        __nanosleep(200);
     }
-    queued = __shfl_sync(0xffffffffu, queued, 0);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (need == 0u) return;
     const unsigned lower = (1u << lane) - 1u;
-    if (queued) {
-        uint32_t first = base, tickets[VPT];
 #pragma unroll
-        for (int j = 0; j < VPT; ++j) {
-            tickets[j] = first + (uint32_t)__popc(bal[j] & lower);
-            first += (uint32_t)__popc(bal[j]);
+    for (int j = 0; j < VPT; ++j) {
+        if ((need >> j) & 1u) {
+            float4 *e = sm.queue_entry(w, ticket + (uint32_t)__popc(bal[j] & lower));
+            float v[4 * ((3 * K + 4) / 4)];
+#pragma unroll
+            for (int i = 0; i < 3 * K; ++i) v[i] = qv[j][i / 3][i % 3];
+            v[3 * K] = __uint_as_float((uint32_t)(o + j));
+#pragma unroll
+            for (int i = 3 * K + 1; i < 4 * ((3 * K + 4) / 4); ++i) v[i] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < (3 * K + 4) / 4; ++k)
+                e[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         }
-#pragma unroll
-        for (int j = 0; j < VPT; ++j) {
-            if (!((need >> j) & 1u)) continue;
-            float *e = sm.queue_entry(w, tickets[j]);
-#pragma unroll
-            for (int i = 0; i < K; ++i) {
-                e[3 * i] = qv[j][i][0];
-                e[3 * i + 1] = qv[j][i][1];
-                e[3 * i + 2] = qv[j][i][2];
-            }
-            e[3 * K] = __int_as_float((int)(o + j));
-        }
-        __threadfence_block();
-#pragma unroll
-        for (int j = 0; j < VPT; ++j)
-            if ((need >> j) & 1u) *sm.queue_seq(w, tickets[j]) = tickets[j] + 1u;
-    } else {
-#pragma unroll
-        for (int j = 0; j < VPT; ++j) {
-            if (!((need >> j) & 1u)) continue;
-            if constexpr (FAST)
-                fast::dual_project<K>(qv[j]);
-            else
-                dual_project<K>(qv[j], thr);
-#pragma unroll
-            for (int i = 0; i < K - 1; ++i)
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    Xout[(3 * i + a) * tp.plane_w + o + j] = Store<ST>::st(qv[j][i][a]);
-        }
+        ticket += (uint32_t)__popc(bal[j]);
     }
+    __syncwarp();
+    if (lane == 0) st_release_cta(sm.q_tail(w), next);
+    return true;
 }
 
 // Everything a launch needs about one volume: tensor maps of both ping-pong
@@ -830,10 +797,9 @@ __device__ __forceinline__ void tiled_item(const TiledSmem<K, R, NT, VPT, ST> &s
                 mbar_init(sm.empty(i), S::MAIN_WARPS + S::HALO_WARPS);
             }
             *abort = 0;
-            for (int w = 0; w < S::NW; ++w) {
+            for (int w = 0; w < S::MAIN_WARPS; ++w) {
                 *sm.q_tail(w) = 0u;
                 *sm.q_head(w) = 0u;
-                *sm.q_done(w) = 0u;
             }
             mbar_fence_init();
         }
@@ -858,7 +824,6 @@ __device__ __forceinline__ void tiled_item(const TiledSmem<K, R, NT, VPT, ST> &s
             float *vb = sm.vb_plane(0);
             for (int i = tid; i < S::D * S::VB_SLOT / 4; i += blockDim.x) vb[i] = 0.0f;
         }
-        for (int i = tid; i < S::NW * S::QN; i += blockDim.x) *sm.queue_seq(i / S::QN, (uint32_t)i) = 0u;
         if (ca - 1 < tp.col_begin) {  // no plane before the first column: its Xi slot reads as zeros
             uint32_t *x0 = reinterpret_cast<uint32_t *>(sm.xi_slot(0));
             for (int i = tid; i < S::XI_SLOT / 4; i += blockDim.x) x0[i] = 0u;
@@ -954,8 +919,8 @@ __device__ __forceinline__ void tiled_item(const TiledSmem<K, R, NT, VPT, ST> &s
                         // dual step at position p-1 once every warp's Vbar of that plane is in
                         ok = mbar_wait_warp(sm.ready(s_prev), ph_prev, abort);
                         if (!ok) break;
-                        stage_b_chunk<K, R, NT, VPT, ST, FAST>(sm, tp, p - 1, s_prev, s_cur, r0, rr, n0, q, tau2, thr,
-                                                         Xout);
+                        ok = stage_b_chunk<K, R, NT, VPT, ST, FAST>(sm, tp, p - 1, s_prev, s_cur, r0, rr, n0, q, tau2,
+                                                                    thr, Xout, abort);
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(sm.empty(s_prev));
@@ -970,14 +935,12 @@ __device__ __forceinline__ void tiled_item(const TiledSmem<K, R, NT, VPT, ST> &s
             if (ok && is_main && c_last == cb - 1) {
                 ok = mbar_wait_warp(sm.ready(s_prev), ph_prev, abort);
                 if (ok)
-                    stage_b_chunk<K, R, NT, VPT, ST, FAST>(sm, tp, P, s_prev, s_cur, r0, rr, n0, q, tau2, thr, Xout);
+                    stage_b_chunk<K, R, NT, VPT, ST, FAST>(sm, tp, P, s_prev, s_cur, r0, rr, n0, q, tau2, thr, Xout,
+                                                           abort);
             }
             if (is_main) {  // this warp queues nothing more (also after an abort)
                 __syncwarp();
-                if (lane == 0) {
-                    __threadfence_block();
-                    atomicAdd(sm.q_done(warp % S::NW), 1u);
-                }
+                if (lane == 0) st_release_cta(sm.q_tail(warp), *sm.q_tail(warp) | kQueueDone);
             }
         }
         // this item's stores (generic proxy) before any later TMA load of them

@@ -443,14 +443,14 @@ template <int K, typename ST>
 int choose_tile(const potts_options &o, TileChoice *tc)
 {
     using TS = ShapesOf<K, ST>;
-    const int d = o.arith == POTTS_ARITH_FAST ? TS::fast : 0;
+    const int d = o.arith == POTTS_ARITH_FAST ? TS::fast : TS::exact;
     tc->rows = TS::r[d];
     tc->slices = TS::t[d];
     tc->vpt = TS::v[d];
     tc->segment = o.segment_cols > 0 ? o.segment_cols : 64;
     if (tc->segment > 64) return fail(POTTS_EINVAL, "segment_cols must be <= 64");
     if (o.tile_rows > 0 || o.tile_slices > 0 || o.tile_vpt > 0) {
-        for (int i = 0; i < TS::n; ++i)
+        for (int i = 0; i < TS::named; ++i)
             if ((o.tile_rows <= 0 || o.tile_rows == TS::r[i]) && (o.tile_slices <= 0 || o.tile_slices == TS::t[i]) &&
                 (o.tile_vpt <= 0 || o.tile_vpt == TS::v[i])) {
                 tc->rows = TS::r[i];

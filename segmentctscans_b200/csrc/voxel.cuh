@@ -26,6 +26,70 @@ struct DykstraThresholds {
 
 __device__ __forceinline__ float fmax_ref(float a, float b) { return (a < b) ? b : a; }
 
+// Dykstra's shrink n = (l - 1) h / l, l = sqrt(s), of a correction vector h with
+// |h|^2 = s, 1 < s, with the bits of the IEEE square root and divisions but none
+// of their branches.  From one reciprocal square root y of s (within 2 ulp, the
+// documented error of rsqrt):
+//   l = RN(sqrt(s))  one Goldschmidt step for sqrt(s) and 1 / (2 sqrt(s)) and a
+//                    correction by the remainder s - g^2;
+//   r = RN(1 / l)    a Newton step from 2 h, but for a few mantissas (its remainder is
+//                    enlarged by an ulp: for the largest mantissa the step ends on a tie);
+//   RN(a / l)        q = RN(a r) is within two ulp, one correction by the
+//                    remainder brings it within one, and the second then gives
+//                    the correctly rounded quotient (P. W. Markstein, IBM J.
+//                    Res. Dev. 34, 1990, and "Software division and square root
+//                    using Goldschmidt's algorithms", 2004).
+// tests/cpp/shrink_check.c runs the first two steps over every mantissa of s and
+// every y within 2 ulp, and the quotients by an exceptional l over every
+// numerator.  The remainders are exact for s up to 2^40 and numerators that are
+// 0 or at least 2^-60 in size; other operands take the operations themselves.
+// (A -0 quotient may come out as +0.)  The branches and the three separate
+// reciprocals of the operations doubled the latency of a Dykstra warp's sweep.
+__device__ __forceinline__ float rsqrt_2ulp(float s)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+    return y;
+}
+// no value is non-zero and below 2^-60 in size (2 bits - 1 wraps a zero to the largest value)
+__device__ __forceinline__ bool none_below_2m60(float a0, float a1, float a2)
+{
+    const uint32_t b0 = __float_as_uint(a0), b1 = __float_as_uint(a1), b2 = __float_as_uint(a2);
+    return min(min(b0 + b0 - 1u, b1 + b1 - 1u), b2 + b2 - 1u) >= (67u << 24) - 1u;
+}
+static __device__ __noinline__ float3 shrink_ops(float h0, float h1, float h2, float s)
+{
+    const float l = __fsqrt_rn(s);
+    const float lm1 = l - 1.0f;
+    return make_float3(__fdiv_rn(lm1 * h0, l), __fdiv_rn(lm1 * h1, l), __fdiv_rn(lm1 * h2, l));
+}
+__device__ __forceinline__ void shrink_rn(float h0, float h1, float h2, float s, float &n0, float &n1, float &n2)
+{
+    const float y = rsqrt_2ulp(s);
+    float g = s * y, h = 0.5f * y;
+    const float e = fmaf(-g, h, 0.5f);
+    g = fmaf(g, e, g);
+    h = fmaf(h, e, h);
+    const float l = fmaf(fmaf(-g, g, s), h, g);
+    const float t = h + h;
+    const float f = fmaf(-l, t, 1.0f);
+    const float r = fmaf(f * 0x1.000002p0f, t, t);
+    const float lm1 = l - 1.0f;
+    const float a0 = lm1 * h0, a1 = lm1 * h1, a2 = lm1 * h2;
+    if (s <= 0x1p40f && none_below_2m60(a0, a1, a2)) {
+        float q0 = a0 * r, q1 = a1 * r, q2 = a2 * r;
+        q0 = fmaf(fmaf(-l, q0, a0), r, q0);
+        q1 = fmaf(fmaf(-l, q1, a1), r, q1);
+        q2 = fmaf(fmaf(-l, q2, a2), r, q2);
+        n0 = fmaf(fmaf(-l, q0, a0), r, q0);
+        n1 = fmaf(fmaf(-l, q1, a1), r, q1);
+        n2 = fmaf(fmaf(-l, q2, a2), r, q2);
+    } else {
+        const float3 n = shrink_ops(h0, h1, h2, s);
+        n0 = n.x, n1 = n.y, n2 = n.z;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Dual step at one voxel (potts-model/potts-min-partition.cpp:96-247):
 //   q = Xi + tau2 * grad+(Vbar), then Dykstra projection onto
@@ -128,11 +192,7 @@ __device__ __forceinline__ bool dykstra_sweep(float (&q)[K][3], float (&P)[K * (
             s = fmaf(h2, h2, s);
             float n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
             if (s > thr.len_gt_one) {
-                const float l = __fsqrt_rn(s);
-                const float lm1 = l - 1.0f;
-                n0 = __fdiv_rn(lm1 * h0, l);
-                n1 = __fdiv_rn(lm1 * h1, l);
-                n2 = __fdiv_rn(lm1 * h2, l);
+                shrink_rn(h0, h1, h2, s, n0, n1, n2);
             }
             const float d0 = 0.5f * (n0 - P[p][0]);
             const float d1 = 0.5f * (n1 - P[p][1]);
@@ -375,6 +435,7 @@ __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
@@ -441,6 +502,75 @@ __device__ __forceinline__ unsigned dual_needs_loop_pair(const float2 (&q)[K][3]
         }
     }
     return (l0 ? 1u : 0u) | (l1 ? 2u : 0u);
+}
+
+// dykstra_sweep of two independent voxels (.x and .y) with the paired
+// instructions; max_dd receives the largest squared step of each.
+template <int K>
+__device__ __forceinline__ void dykstra_sweep_pair(float2 (&q)[K][3], float2 (&P)[K * (K - 1) / 2][3],
+                                                   DykstraThresholds thr, float2 &max_dd)
+{
+    max_dd = f2(0.0f);
+    int p = 0;
+#pragma unroll
+    for (int i1 = 0; i1 < K - 1; ++i1) {
+#pragma unroll
+        for (int i2 = i1 + 1; i2 < K; ++i2, ++p) {
+            float2 h[3], n[3], d[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) h[a] = add2(sub2(q[i2][a], q[i1][a]), P[p][a]);
+            const float2 s = fma2(h[2], h[2], fma2(h[1], h[1], mul2(h[0], h[0])));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) n[a] = f2(0.0f);
+            // both voxels at once; one whose pair is not longer than 1 runs with s = 1, whose
+            // l - 1 and so its n are 0
+            const bool x = s.x > thr.len_gt_one, y = s.y > thr.len_gt_one;
+            if (x || y) {
+                const float2 s1 = f2(x ? s.x : 1.0f, y ? s.y : 1.0f);
+                const float2 rs = f2(rsqrt_2ulp(s1.x), rsqrt_2ulp(s1.y));  // shrink_rn
+                float2 g = mul2(s1, rs), z = mul2(f2(0.5f), rs);
+                const float2 e = fma2(neg2(g), z, f2(0.5f));
+                g = fma2(g, e, g);
+                z = fma2(z, e, z);
+                const float2 l = fma2(fma2(neg2(g), g, s1), z, g), ml = neg2(l);
+                const float2 t = add2(z, z);
+                const float2 f = fma2(ml, t, f2(1.0f));
+                const float2 r = fma2(mul2(f, f2(0x1.000002p0f)), t, t);
+                const float2 lm1 = add2(l, f2(-1.0f));
+                float2 m[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) m[a] = mul2(lm1, h[a]);
+                if (s.x <= 0x1p40f && s.y <= 0x1p40f && none_below_2m60(m[0].x, m[1].x, m[2].x) &&
+                    none_below_2m60(m[0].y, m[1].y, m[2].y)) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        float2 v = mul2(m[a], r);
+                        v = fma2(fma2(ml, v, m[a]), r, v);
+                        n[a] = fma2(fma2(ml, v, m[a]), r, v);
+                    }
+                } else {
+                    if (x) {
+                        const float3 w = shrink_ops(h[0].x, h[1].x, h[2].x, s.x);
+                        n[0].x = w.x, n[1].x = w.y, n[2].x = w.z;
+                    }
+                    if (y) {
+                        const float3 w = shrink_ops(h[0].y, h[1].y, h[2].y, s.y);
+                        n[0].y = w.x, n[1].y = w.y, n[2].y = w.z;
+                    }
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) d[a] = mul2(f2(0.5f), sub2(n[a], P[p][a]));
+            const float2 dd = fma2(d[2], d[2], fma2(d[1], d[1], mul2(d[0], d[0])));
+            max_dd = f2(fmax_ref(dd.x, max_dd.x), fmax_ref(dd.y, max_dd.y));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                q[i1][a] = add2(q[i1][a], d[a]);
+                q[i2][a] = sub2(q[i2][a], d[a]);
+                P[p][a] = n[a];
+            }
+        }
+    }
 }
 
 template <int K>

@@ -20,7 +20,8 @@
 //     it), for K = 2, 3 without sorting, with multiplications by constant
 //     reciprocals;
 //   * Dykstra's shrink (l - 1) h / l is h (1 - rsqrt(s)), s = |h|^2, and the
-//     exit test sqrt(max |delta|^2) < 1e-6 is max |delta|^2 < 1e-12.
+//     exit test sqrt(max |delta|^2) < 1e-6 is max |2 delta|^2 < 4e-12; the
+//     halving of a step is part of the multiply-add that applies it.
 // Every function is written once for F = float (one voxel) and F = float2
 // (two consecutive slices with Blackwell's paired FP32 instructions); the two
 // lanes of a pair run exactly the operations of the scalar form, so the split
@@ -29,6 +30,8 @@
 #pragma once
 
 #include <cstdint>
+
+#include "voxel.cuh"
 
 namespace potts {
 namespace fast {
@@ -204,39 +207,45 @@ __device__ __forceinline__ F max_pair_dist2(const F (&q)[K][3])
     return m;
 }
 
-// One sweep of Dykstra's loop over the pairs (i1 < i2); true when the loop
-// exits after it (every correction step shorter than 1e-6).
-template <int K>
-__device__ __forceinline__ bool dykstra_sweep(float (&q)[K][3], float (&P)[K * (K - 1) / 2][3])
+// 1 - 1/|h| where |h|^2 = s exceeds 1, else 0 (a normal s: rsqrt's subnormal handling is not needed).
+__device__ __forceinline__ float shrink(float s) { return s > 1.0f ? sub(1.0f, rsqrt_2ulp(s)) : 0.0f; }
+__device__ __forceinline__ float2 shrink(float2 s) { return make_float2(shrink(s.x), shrink(s.y)); }
+__device__ __forceinline__ float max_of(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ float2 max_of(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+
+// One sweep of Dykstra's loop over the pairs (i1 < i2) of one voxel or of two
+// independent ones.  Returns the largest squared length of twice a correction
+// step, e = n - P = 2 delta (the loop exits after a sweep whose steps are all
+// shorter than 1e-6: below kExit2).
+constexpr float kExit2 = 4.0f * 1e-12f;
+template <int K, typename F>
+__device__ __forceinline__ F dykstra_sweep(F (&q)[K][3], F (&P)[K * (K - 1) / 2][3])
 {
-    float max_dd = 0.0f;
+    F step = splat<F>(0.0f);
     int p = 0;
 #pragma unroll
     for (int i1 = 0; i1 < K - 1; ++i1) {
 #pragma unroll
         for (int i2 = i1 + 1; i2 < K; ++i2, ++p) {
-            const float h0 = add(sub(q[i2][0], q[i1][0]), P[p][0]);
-            const float h1 = add(sub(q[i2][1], q[i1][1]), P[p][1]);
-            const float h2 = add(sub(q[i2][2], q[i1][2]), P[p][2]);
-            const float s = fma(h2, h2, fma(h1, h1, mul(h0, h0)));
-            const float f = s > 1.0f ? sub(1.0f, rsqrtf(s)) : 0.0f;
-            const float n0 = mul(h0, f), n1 = mul(h1, f), n2 = mul(h2, f);
-            const float d0 = mul(0.5f, sub(n0, P[p][0]));
-            const float d1 = mul(0.5f, sub(n1, P[p][1]));
-            const float d2 = mul(0.5f, sub(n2, P[p][2]));
-            max_dd = fmaxf(max_dd, fma(d2, d2, fma(d1, d1, mul(d0, d0))));
-            q[i1][0] = add(q[i1][0], d0);
-            q[i1][1] = add(q[i1][1], d1);
-            q[i1][2] = add(q[i1][2], d2);
-            q[i2][0] = sub(q[i2][0], d0);
-            q[i2][1] = sub(q[i2][1], d1);
-            q[i2][2] = sub(q[i2][2], d2);
-            P[p][0] = n0;
-            P[p][1] = n1;
-            P[p][2] = n2;
+            F h[3], e[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) h[a] = add(sub(q[i2][a], q[i1][a]), P[p][a]);
+            const F f = shrink(fma(h[2], h[2], fma(h[1], h[1], mul(h[0], h[0]))));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const F n = mul(h[a], f);
+                e[a] = sub(n, P[p][a]);
+                P[p][a] = n;
+            }
+            step = max_of(step, fma(e[2], e[2], fma(e[1], e[1], mul(e[0], e[0]))));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                q[i1][a] = fma(splat<F>(0.5f), e[a], q[i1][a]);
+                q[i2][a] = fma(splat<F>(-0.5f), e[a], q[i2][a]);
+            }
         }
     }
-    return max_dd < 1e-12f;
+    return step;
 }
 
 // The whole projection loop from zero corrections (at most 20 sweeps).
@@ -248,7 +257,7 @@ __device__ __forceinline__ void dual_project(float (&q)[K][3])
 #pragma unroll
     for (int p = 0; p < kPairs; ++p) P[p][0] = P[p][1] = P[p][2] = 0.0f;
     for (int sweeps = 1; sweeps <= 20; ++sweeps)
-        if (dykstra_sweep<K>(q, P)) break;
+        if (dykstra_sweep<K, float>(q, P) < kExit2) break;
 }
 
 }  // namespace fast
