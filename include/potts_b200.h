@@ -103,10 +103,10 @@ typedef struct potts_options {
     int slab_w;       /* 0: plan slabs from free memory like the reference; > 0: force this slab width */
     int track_dq;     /* 1: record max_x |V^{k+1} - V^k|^2 of every iteration on the device */
     int sync_monitor; /* 1: reference behaviour, read the monitor back and sync after every iteration */
-    int tile_rows;    /* fused form: rows per tile (0 = default for K and arith) */
-    int tile_slices;  /* fused form: slices (n) per tile (0 = default for K) */
-    int segment_cols; /* fused form: columns one tile marches over (0 = 64, at most 64) */
-    int tile_vpt;     /* fused form: consecutive slices per thread, 2 or 4 (0 = default for K) */
+    int tile_rows;    /* fused form: rows per tile (0 = chosen by K, arith and the volume's size) */
+    int tile_slices;  /* fused form: slices (n) per tile (0 = chosen likewise) */
+    int segment_cols; /* fused form: columns one tile marches over (0 = chosen by the volume's size, at most 64) */
+    int tile_vpt;     /* fused form: consecutive slices per thread, 2 or 4 (0 = chosen likewise) */
     int prefetch;     /* fused form: planes the load ring prefetches into L2 ahead of its loads
                          (0 = default: none, < 0 = none, at most 16) */
     int autotune;     /* batches: 1 = time every compiled tile shape and segment length, each as one

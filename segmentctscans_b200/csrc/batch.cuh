@@ -323,7 +323,10 @@ int batch_build(potts_batch *b)
         b->iters > 1) {
         POTTS_TRY((batch_autotune<K, ST>(b, &tile, &b->opts.persistent)));
     } else {
-        POTTS_TRY((choose_tile<K, ST>(o, &tile)));
+        std::vector<MarchVolume> vols;
+        for (const BatchVolume &bv : b->vols)
+            vols.push_back({&bv.mc.m, bv.g.ns, (int)bv.mc.m.col_begin, (int)bv.mc.m.col_end});
+        POTTS_TRY((choose_tile<K, ST>(o, vols, ctx->n_sm, &tile)));
     }
     POTTS_TRY((batch_plan_tiles<K, ST>(b, tile)));
     // the kernel's shared-memory attribute is set (and the persistent launch's

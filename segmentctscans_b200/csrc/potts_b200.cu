@@ -12,7 +12,9 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <type_traits>
+#include <utility>
 #include <string>
 #include <vector>
 
@@ -187,6 +189,11 @@ bool same_mapping(const MappingCopy &a, const potts_mapping &b)
            std::memcmp(a.base.data(), b.base, sizeof(uint32_t) * (b.cols + 1)) == 0;
 }
 
+// Tile shape and column segment of a march kernel's work items.
+struct TileChoice {
+    int rows, slices, vpt, segment;
+};
+
 // Grow-only device buffer owned by a context.
 struct DevBuf {
     void *p = nullptr;
@@ -214,6 +221,10 @@ struct potts_context {
     int n_sm = 0;  // multiprocessors of the device
     bool cols_valid = false;
     int work_key[5] = {-1, -1, -1, -1, -1};
+    // the fused kernel's tile for this mapping and the key's slab width and options
+    TileChoice tile{};
+    int tile_key[8] = {};
+    bool tile_valid = false;
     int gm_segment = 0, gm_ns = -1;  // grad_magn's column segment for this mapping and slice count
     int n_work = 0;
     // Event pairs around runs of consecutive iteration launches (energy
@@ -309,6 +320,7 @@ int upload_lines(potts_context *ctx, const potts_mapping *map)
     ctx->mapping_valid = false;
     ctx->cols_valid = false;
     ctx->work_key[0] = -1;
+    ctx->tile_valid = false;
     ctx->gm_segment = 0;
     POTTS_TRY(copy_mapping(map, ctx->mapping));
     const size_t bytes = sizeof(int4) * (size_t)std::max<int64_t>(ctx->mapping.n_lines, 1);
@@ -435,32 +447,135 @@ int encode_map(CUtensorMap *m, CUtensorMapDataType dt, const void *base, int ran
 // (none: prefetching 2 or 4 planes measured 0.5-3 % slower at 768^2 x 1024).
 constexpr int kDefaultPrefetch = 0;
 
-struct TileChoice {
-    int rows, slices, vpt, segment;
+// The slices and columns that a column-march kernel runs over.
+struct MarchVolume {
+    const potts_mapping *map;
+    int ns;
+    int c_begin, c_end;
 };
 
+// Columns [first, second) of a run of columns that hold a tile's rows.
+using ColumnRun = std::pair<int, int>;
+
+std::vector<ColumnRun> tile_runs(const potts_mapping &m, int r0, int rows, int c_begin, int c_end)
+{
+    std::vector<ColumnRun> runs;
+    for (int c = c_begin; c < c_end; ++c) {
+        const int64_t cnt = (int64_t)(m.base[c + 1] - m.base[c]) / m.nstride;
+        if (cnt <= 0 || (int64_t)m.start_row[c] >= r0 + rows || (int64_t)m.start_row[c] + cnt <= r0) continue;
+        if (!runs.empty() && runs.back().second == c)
+            runs.back().second = c + 1;
+        else
+            runs.push_back({c, c + 1});
+    }
+    return runs;
+}
+
+// First row and one past the last row of the columns [c_begin, c_end).
+std::pair<int, int> row_range(const potts_mapping &m, int c_begin, int c_end)
+{
+    int lo = INT32_MAX, hi = 0;
+    for (int c = c_begin; c < c_end; ++c) {
+        const int64_t cnt = (int64_t)(m.base[c + 1] - m.base[c]) / m.nstride;
+        if (cnt <= 0) continue;
+        lo = std::min<int>(lo, (int)m.start_row[c]);
+        hi = std::max<int>(hi, (int)(m.start_row[c] + cnt));
+    }
+    return {lo, hi};
+}
+
+// Column planes that a work item costs besides those of its columns: the plane
+// before and after them, filling the load ring and the drain at its end.  With
+// 4 the choice below was within 2 % (at most 9 %) of the best of 13 segment
+// lengths on cores of 128^3 to 203 x 301 x 287 voxels, three shapes and both arithmetics.
+constexpr int kItemPlanes = 4;
+constexpr int kSegments[] = {64, 48, 40, 32, 24, 20, 16, 12, 10, 8, 6};
+
+// Expected time of the volumes' work items for rows x slices tiles (in planes of
+// one tile), and the segment length that gives it (`segment` > 0: that one).  A
+// block runs one item and `slots` blocks run at a time, so a volume of few tiles
+// leaves multiprocessors idle, or its last wave nearly empty, with long segments,
+// and pays kItemPlanes too often with short ones: 128^3 (radius 60, fast, 8 x
+// 128 tiles) takes 171 us per iteration with segments of 64 columns (30 items), 52
+// with 10 and 57 with 4.  The items go to the first free slot in order, as the
+// hardware hands out blocks; with at least kManyWaves items per slot their mean decides.
+constexpr int kManyWaves = 12;
+double march_time(const std::vector<MarchVolume> &vols, int rows, int slices, int slots, int segment, int *best)
+{
+    struct Run {
+        int len, tiles;
+    };
+    std::vector<Run> runs;
+    for (const MarchVolume &v : vols) {
+        const auto [lo, hi] = row_range(*v.map, v.c_begin, v.c_end);
+        const int tiles = (v.ns + slices - 1) / slices;
+        for (int r0 = lo; r0 < hi; r0 += rows)
+            for (const ColumnRun &r : tile_runs(*v.map, r0, rows, v.c_begin, v.c_end))
+                runs.push_back({r.second - r.first, tiles});
+    }
+    double best_time = -1.0;
+    std::vector<int> ends, lens;
+    for (int seg : kSegments) {
+        if (segment > 0) seg = segment;
+        int64_t items = 0, planes = 0;
+        int longest = 0;
+        for (const Run &r : runs) {
+            const int n = (r.len + seg - 1) / seg;
+            items += (int64_t)n * r.tiles;
+            planes += (int64_t)(r.len + n * kItemPlanes) * r.tiles;
+            longest = std::max(longest, (r.len + seg - 1) / seg);
+        }
+        double time = (double)planes / slots;
+        if (items < (int64_t)kManyWaves * slots && (best_time < 0.0 || time < best_time)) {
+            lens.clear();
+            for (int k = 0; k < longest; ++k)
+                for (const Run &r : runs)
+                    if (k * seg < r.len) lens.insert(lens.end(), (size_t)r.tiles, std::min(seg, r.len - k * seg));
+            ends.assign((size_t)slots, 0);  // a heap, the first free slot on top
+            for (int len : lens) {
+                std::pop_heap(ends.begin(), ends.end(), std::greater<int>());
+                ends.back() += len + kItemPlanes;
+                std::push_heap(ends.begin(), ends.end(), std::greater<int>());
+            }
+            time = (double)*std::max_element(ends.begin(), ends.end());
+        }
+        if (best_time < 0.0 || time < best_time) {
+            best_time = time;
+            *best = seg;
+        }
+        // many items with the longest segments: shorter ones only add planes
+        if (segment > 0 || (seg == kSegments[0] && items >= (int64_t)kManyWaves * slots)) break;
+    }
+    return best_time;
+}
+
+// Tile shape and segment length: the options', or those with the least expected
+// time over the volumes (a shape's time per voxel times its march_time: ragged
+// slices and rows cost as much as full ones).  The results depend on neither.
 template <int K, typename ST>
-int choose_tile(const potts_options &o, TileChoice *tc)
+int choose_tile(const potts_options &o, const std::vector<MarchVolume> &vols, int n_sm, TileChoice *tc)
 {
     using TS = ShapesOf<K, ST>;
-    const int d = o.arith == POTTS_ARITH_FAST ? TS::fast : TS::exact;
-    tc->rows = TS::r[d];
-    tc->slices = TS::t[d];
-    tc->vpt = TS::v[d];
-    tc->segment = o.segment_cols > 0 ? o.segment_cols : 64;
-    if (tc->segment > 64) return fail(POTTS_EINVAL, "segment_cols must be <= 64");
-    if (o.tile_rows > 0 || o.tile_slices > 0 || o.tile_vpt > 0) {
-        for (int i = 0; i < TS::named; ++i)
-            if ((o.tile_rows <= 0 || o.tile_rows == TS::r[i]) && (o.tile_slices <= 0 || o.tile_slices == TS::t[i]) &&
-                (o.tile_vpt <= 0 || o.tile_vpt == TS::v[i])) {
-                tc->rows = TS::r[i];
-                tc->slices = TS::t[i];
-                tc->vpt = TS::v[i];
-                return POTTS_OK;
-            }
+    if (o.segment_cols > 64) return fail(POTTS_EINVAL, "segment_cols must be <= 64");
+    const bool named = o.tile_rows > 0 || o.tile_slices > 0 || o.tile_vpt > 0;
+    double best = -1.0;
+    for (int i = 0; i < (named ? TS::named : TS::n); ++i) {
+        if (named && !((o.tile_rows <= 0 || o.tile_rows == TS::r[i]) && (o.tile_slices <= 0 || o.tile_slices == TS::t[i]) &&
+                       (o.tile_vpt <= 0 || o.tile_vpt == TS::v[i])))
+            continue;
+        int segment = 64;
+        const int weight = o.arith == POTTS_ARITH_FAST ? TS::fast[i] : TS::exact[i];
+        const double time = march_time(vols, TS::r[i], TS::t[i], std::max(n_sm, 1), o.segment_cols, &segment) *
+                            (weight * TS::r[i] * TS::t[i]);
+        if (best < 0.0 || time < best) {
+            best = time;
+            *tc = TileChoice{TS::r[i], TS::t[i], TS::v[i], segment};
+        }
+        if (named) break;  // the first shape that matches
+    }
+    if (best < 0.0)
         return fail(POTTS_EINVAL,
                     "tile_rows x tile_slices x tile_vpt is not a compiled tile shape for this K and storage");
-    }
     return POTTS_OK;
 }
 
@@ -484,36 +599,19 @@ std::vector<int4> column_table(const potts_mapping &m)
 std::vector<int4> work_items(const potts_mapping &m, int ns, const TileChoice &tc, int c_begin = -1, int c_end = -1)
 {
     // the columns [c_begin, c_end) (default: all active columns)
-    const uint32_t cb0 = c_begin < 0 ? m.col_begin : (uint32_t)c_begin;
-    const uint32_t ce0 = c_end < 0 ? m.col_end : (uint32_t)c_end;
-    int row_lo = INT32_MAX, row_hi = 0;
-    for (uint32_t c = cb0; c < ce0; ++c) {
-        const int64_t cnt = (int64_t)(m.base[c + 1] - m.base[c]) / m.nstride;
-        if (cnt <= 0) continue;
-        row_lo = std::min<int>(row_lo, (int)m.start_row[c]);
-        row_hi = std::max<int>(row_hi, (int)(m.start_row[c] + cnt));
-    }
+    const int cb0 = c_begin < 0 ? (int)m.col_begin : c_begin;
+    const int ce0 = c_end < 0 ? (int)m.col_end : c_end;
+    const auto [row_lo, row_hi] = row_range(m, cb0, ce0);
     struct Item {
         int ca, r0, n0, cb;
     };
     std::vector<Item> items;
     const int tiles = (ns + tc.slices - 1) / tc.slices;
-    for (int r0 = row_lo; r0 < row_hi; r0 += tc.rows) {
-        int run = -1;
-        for (int c = (int)cb0; c <= (int)ce0; ++c) {
-            bool active = false;
-            if (c < (int)ce0) {
-                const int64_t cnt = (int64_t)(m.base[c + 1] - m.base[c]) / m.nstride;
-                active = cnt > 0 && (int)m.start_row[c] < r0 + tc.rows && (int)(m.start_row[c] + cnt) > r0;
-            }
-            if (active && run < 0) run = c;
-            if (!active && run >= 0) {
-                for (int ca = run; ca < c; ca += tc.segment)
-                    for (int t = 0; t < tiles; ++t) items.push_back({ca, r0, t * tc.slices, std::min(c, ca + tc.segment)});
-                run = -1;
-            }
-        }
-    }
+    for (int r0 = row_lo; r0 < row_hi; r0 += tc.rows)
+        for (const ColumnRun &run : tile_runs(m, r0, tc.rows, cb0, ce0))
+            for (int ca = run.first; ca < run.second; ca += tc.segment)
+                for (int t = 0; t < tiles; ++t)
+                    items.push_back({ca, r0, t * tc.slices, std::min(run.second, ca + tc.segment)});
     std::sort(items.begin(), items.end(), [](const Item &a, const Item &b) {
         if (a.ca != b.ca) return a.ca < b.ca;
         if (a.r0 != b.r0) return a.r0 < b.r0;
@@ -687,7 +785,17 @@ template <int K, typename ST>
 int prepare_fused(potts_context *ctx, const Geometry &g, const ST *const xi[2], const ST *const v[2],
                   const float *d_u, const potts_options &o, const PhaseParams<K> &pp, float *dq, FusedPlan<K, ST> *fp)
 {
-    POTTS_TRY((choose_tile<K, ST>(o, &fp->tile)));
+    // chosen once per mapping, slab width and options
+    const int key[8] = {K, o.storage, o.arith, g.ns, o.tile_rows, o.tile_slices, o.tile_vpt, o.segment_cols};
+    if (!ctx->tile_valid || !std::equal(key, key + 8, ctx->tile_key)) {
+        const potts_mapping &m = ctx->mapping.m;
+        TileChoice tc{};
+        POTTS_TRY((choose_tile<K, ST>(o, {{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, ctx->n_sm, &tc)));
+        std::copy(key, key + 8, ctx->tile_key);
+        ctx->tile = tc;
+        ctx->tile_valid = true;
+    }
+    fp->tile = ctx->tile;
     POTTS_TRY(plan_tiles(ctx, g.ns, fp->tile));
     fp->n_work = ctx->n_work;
     const float *ubase;

@@ -223,14 +223,14 @@ Geometry shard_geometry(const potts_shard *s)
 size_t store_bytes(int storage) { return storage == POTTS_STORE_F32 ? 4 : 2; }
 
 template <typename ST>
-int choose_tile_k(int K, const potts_options &o, TileChoice *tc)
+int choose_tile_k(int K, const potts_options &o, const std::vector<MarchVolume> &vols, int n_sm, TileChoice *tc)
 {
     switch (K) {
-    case 2: return choose_tile<2, ST>(o, tc);
-    case 3: return choose_tile<3, ST>(o, tc);
-    case 4: return choose_tile<4, ST>(o, tc);
-    case 5: return choose_tile<5, ST>(o, tc);
-    case 6: return choose_tile<6, ST>(o, tc);
+    case 2: return choose_tile<2, ST>(o, vols, n_sm, tc);
+    case 3: return choose_tile<3, ST>(o, vols, n_sm, tc);
+    case 4: return choose_tile<4, ST>(o, vols, n_sm, tc);
+    case 5: return choose_tile<5, ST>(o, vols, n_sm, tc);
+    case 6: return choose_tile<6, ST>(o, vols, n_sm, tc);
     }
     return fail(POTTS_EINVAL, "K must be in [2, 6]");
 }
@@ -279,13 +279,14 @@ int shard_create(potts_context *ctx, const potts_mapping *map, const uint32_t *c
     POTTS_CUDA(cudaMemcpy(s->cols.p, cols.data(), sizeof(int4) * cols.size(), cudaMemcpyHostToDevice));
     // tile and work items: the owned columns and, with a right neighbour, its first column
     // (the primal step there gives Vbar and V at b; see the top of this file)
-    switch (o.storage) {
-    case POTTS_STORE_BF16: POTTS_TRY(choose_tile_k<__nv_bfloat16>(K, o, &s->tile)); break;
-    case POTTS_STORE_F16: POTTS_TRY(choose_tile_k<__half>(K, o, &s->tile)); break;
-    default: POTTS_TRY(choose_tile_k<float>(K, o, &s->tile)); break;
-    }
     const uint32_t a = shard_local_col(s.get(), sc.own_begin);
     const uint32_t b1 = std::min<uint32_t>(shard_local_col(s.get(), sc.own_end) + 1, s->mc.m.cols);
+    const std::vector<MarchVolume> vols = {{&s->mc.m, (int)lm.n_images, (int)a, (int)b1}};
+    switch (o.storage) {
+    case POTTS_STORE_BF16: POTTS_TRY(choose_tile_k<__nv_bfloat16>(K, o, vols, ctx->n_sm, &s->tile)); break;
+    case POTTS_STORE_F16: POTTS_TRY(choose_tile_k<__half>(K, o, vols, ctx->n_sm, &s->tile)); break;
+    default: POTTS_TRY(choose_tile_k<float>(K, o, vols, ctx->n_sm, &s->tile)); break;
+    }
     const std::vector<int4> work = work_items(s->mc.m, (int)lm.n_images, s->tile, (int)a, (int)b1);
     POTTS_TRY(ensure(ctx, s->work, sizeof(int4) * std::max<size_t>(work.size(), 1)));
     if (!work.empty())
