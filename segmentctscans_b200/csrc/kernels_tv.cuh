@@ -15,6 +15,7 @@
 #include "geometry.cuh"
 #include "kernels_plain.cuh"
 #include "tma.cuh"
+#include "voxel.cuh"
 
 namespace potts {
 
@@ -146,243 +147,336 @@ __global__ void __launch_bounds__(kPlainThreads) tv_update_kernel(Geometry g, fl
     gio[o] = fmaf(-lam, tv_div_at(g, xi, o, p.n, li), gio[o]);
 }
 
-// The lambda-scaled forward differences of g that grad_kernel (:89-166) computes in every
-// iteration, computed once per solve with the same operations: D_n = (g(x+e_n) - g(x)) /
-// lambda, D_r and D_c likewise (zero where the neighbour does not exist), three planes laid
-// out like g.  g does not change during the iterations, so an iteration that reads D gets
-// the same bits as one that recomputes it.
-__global__ void __launch_bounds__(kPlainThreads) tv_gdiff_kernel(Geometry g, const float *__restrict__ gin,
-                                                                 float *__restrict__ D, float lam)
+// Whether every forward difference of g is 0 or between 2^-60 and 2^60 in size (*unsafe is set
+// where one is not): the quotients by lambda then come from its reciprocal (div4_rn).
+__global__ void __launch_bounds__(kPlainThreads) tv_range_kernel(Geometry g, const float *__restrict__ gin,
+                                                                 int *__restrict__ unsafe)
 {
     const PlainIndex p = plain_index(g, 0, g.ns);
     if (!p.valid) return;
     const LineInfo li = load_line(g, p.line);
     const int64_t o = p.line * g.nstride_w + p.n;
+    const float g0 = gin[o];
     float d1 = 0.0f, d2 = 0.0f, d3 = 0.0f;
-    if (p.n + 1 < g.ns) d1 = __fdiv_rn(gin[o + 1] - gin[o], lam);
-    if (li.flags & kHasNextRow) d2 = __fdiv_rn(gin[o + g.nstride_w] - gin[o], lam);
-    if (li.next_col >= 0) d3 = __fdiv_rn(gin[(int64_t)li.next_col * g.nstride_w + p.n] - gin[o], lam);
-    D[o] = d1;
-    D[g.plane_w + o] = d2;
-    D[2 * g.plane_w + o] = d3;
+    if (p.n + 1 < g.ns) d1 = gin[o + 1] - g0;
+    if (li.flags & kHasNextRow) d2 = gin[o + g.nstride_w] - g0;
+    if (li.next_col >= 0) d3 = gin[(int64_t)li.next_col * g.nstride_w + p.n] - g0;
+    if (!none_below_2m60(d1, d2, d3) || !(fabsf(d1) <= 0x1p60f) || !(fabsf(d2) <= 0x1p60f) ||
+        !(fabsf(d3) <= 0x1p60f))
+        *unsafe = 1;
 }
 
-}  // namespace potts
-
-namespace potts {
-
-// Tiled fused iteration.  A block owns a tile of TR rows x TN slices and marches
+// Tiled fused iteration.  A block owns a tile of 8 rows x 128 slices and marches
 // over the columns [ca, cb) of its work item (x = first row, y = first slice,
-// z/w = column range, the work items of the Potts kernel).  Shared memory holds
-// a ring of three column planes of xi (rows r0-1 .. r0+TR, slices n0-4 ..
-// n0+TN+3, the three components), each one TMA box loaded two planes ahead of
-// the plane being updated, and two planes of v = div xi (rows r0 .. r0+TR,
-// slices n0 .. n0+TN), so that each xi value is read from DRAM once per plane
-// and v is computed once per voxel.  The lambda-scaled differences of g come
-// from tv_gdiff_kernel's planes.  The operations per voxel are those of
-// tv_div_at and tv_grad_kernel, in the same order.  The xi box starts at slice
-// n0-4 so that its first word is 16-byte aligned: slice n sits at n - n0 + 4 of
-// a row (stride TN + 8); v rows hold slice n at n - n0 (stride TN + 4).  Box
-// rows outside the plane's column come from other columns or are zero-filled;
-// they are never read.
-template <int TR, int TN>
+// z/w = column range).  Warp w < 8 owns row r0 + w and each of its lanes four
+// consecutive slices, so every condition on rows and columns is the same in a
+// whole warp and shared memory is read 16 bytes at a time; warp 8 computes what
+// the tile needs of v = div xi on row r0 + 8 and at slice n0 + 128.  Shared
+// memory holds a ring of three column planes of xi (rows r0-1 .. r0+8, slices
+// n0-4 .. n0+131, the three components), each one TMA box, and two planes of v,
+// from which a warp reads the row below; v of a lane's own voxels at the planes c
+// and c+1, and g at c, c+1 and on the row below, stay in its registers (g is
+// loaded a plane ahead).  One barrier per plane.  The operations per voxel are
+// those of tv_div_at and tv_grad_kernel, in the same order and with the same
+// rounding: two slices at a time with the paired instructions, quotients by one
+// divisor from its reciprocal where the remainders are exact (for lambda and the
+// differences of g that is known before the first iteration).  Box rows outside the plane's column come from other columns or are
+// zero-filled; their values are never used.
+// HBM traffic per voxel and iteration: xi in and out, g in (28 bytes; three planes
+// of precomputed differences of g / lambda in place of g cost 36).  At 512 x 512 x
+// 512 (radius 246) an iteration takes 0.61 ms (4.5 TB/s; 0.79 ms with one slice and
+// four rows per thread, scalar arithmetic and the difference planes): 4.0 warp
+// instructions per voxel at 59 % of the issue slots.  Two blocks of 96 registers
+// per multiprocessor: with three (72 registers) it spills, 0.75 ms.
 struct TvTile {
-    static_assert(TN % 4 == 0, "16-byte aligned box start");
-    static constexpr int XR = TR + 2, XS = TN + 8;  // xi box: rows r0-1 .., row stride
-    static constexpr int VR = TR + 1, GS = TN + 4;  // v box: rows r0 .., row stride
+    static constexpr int TR = 8, TN = 128, SLOTS = 3;
+    static constexpr int XR = TR + 2, XS = TN + 8;  // xi box: rows r0-1 .., row stride (slice n at n - n0 + 4)
+    static constexpr int VR = TR + 1, VS = TN + 4;  // v plane: rows r0 .., row stride (slice n at n - n0)
     static constexpr int XC = XR * XS;              // one xi component
     static constexpr int XI_PLANE = 3 * XC;
     static constexpr int XI_SLOT = (XI_PLANE + 31) / 32 * 32;  // 128-byte aligned slots
-    static constexpr int V_PLANE = VR * GS;
+    static constexpr int V_PLANE = VR * VS;
     static constexpr uint32_t BOX_BYTES = 4u * XI_PLANE;
-    static constexpr int OFF_BAR = 4 * (3 * XI_SLOT + 2 * V_PLANE);  // bytes: 3 mbarriers, abort flag
-    static constexpr int SMEM_BYTES = OFF_BAR + 3 * 8 + 8 + 128;     // + alignment slack
+    static constexpr int OFF_BAR = 4 * (SLOTS * XI_SLOT + 2 * V_PLANE);  // bytes: mbarriers, abort flag
+    static constexpr int SMEM_BYTES = OFF_BAR + SLOTS * 8 + 8 + 128;     // + alignment slack
 };
+constexpr int kTvThreads = 32 * (TvTile::TR + 1);
+constexpr int kTvBlocks = 2;  // per multiprocessor
 
 // column table entry: x = first line, y/z = row range of the column (the Potts kernel's table)
 __device__ __forceinline__ bool tv_row_in(int4 ci, int row) { return row >= ci.y && row < ci.z; }
 
-}  // namespace potts
+// Four values as two pairs.
+struct Quad {
+    float2 a, b;
+};
+__device__ __forceinline__ Quad quad(float4 v) { return Quad{f2(v.x, v.y), f2(v.z, v.w)}; }
+__device__ __forceinline__ Quad lds4(const float *p) { return quad(*reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ Quad zero4() { return Quad{f2(0.0f), f2(0.0f)}; }
+__device__ __forceinline__ Quad add4(Quad x, Quad y) { return Quad{add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ Quad sub4(Quad x, Quad y) { return Quad{sub2(x.a, y.a), sub2(x.b, y.b)}; }
+// x with the elements j where m has no bit j set to 0
+__device__ __forceinline__ Quad keep4(Quad x, unsigned m)
+{
+    return Quad{f2(m & 1u ? x.a.x : 0.0f, m & 2u ? x.a.y : 0.0f), f2(m & 4u ? x.b.x : 0.0f, m & 8u ? x.b.y : 0.0f)};
+}
+// x / b, correctly rounded, from the correctly rounded reciprocal r of b (in_range: 2^-20 <= |b| <=
+// 2^20 and x is 0 or between 2^-60 and 2^60 in size, see shrink_rn)
+__device__ __forceinline__ Quad div4_rn(Quad x, float b, float r, bool in_range)
+{
+    if (in_range) return Quad{quot2_rn(x.a, f2(-b), f2(r)), quot2_rn(x.b, f2(-b), f2(r))};
+    return Quad{f2(__fdiv_rn(x.a.x, b), __fdiv_rn(x.a.y, b)), f2(__fdiv_rn(x.b.x, b), __fdiv_rn(x.b.y, b))};
+}
 
-namespace potts {
+__device__ __forceinline__ float rcp_1ulp(float b)  // 1 / b, b normal
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
 
-constexpr int kTvThreads = 256;
+// xi <- (xi + tau G) / (1 + tau |G|) for four voxels; returns |dxi|^2 of each.  With 0 <= tau <= 1
+// (tau_in_range), |G|^2 <= 2^40 and no tiny numerators the root and the quotients are those of shrink_rn:
+// |G|^2 below 2^-80 gives a denominator of 1 whatever its root, so it is raised to that.  Else the IEEE
+// operations run (the same bits).
+__device__ __forceinline__ uint32_t below_key(float2 a)  // none_below_2m60's key of two values
+{
+    const uint32_t x = __float_as_uint(a.x), y = __float_as_uint(a.y);
+    return min(x + x - 1u, y + y - 1u);
+}
+__device__ __forceinline__ Quad tv_step(Quad (&x)[3], const Quad (&G)[3], float tau, bool tau_in_range)
+{
+    const float2 t = f2(tau);
+    float2 s[2], a[2][3], q[2][3], d[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float2 g0 = h ? G[0].b : G[0].a, g1 = h ? G[1].b : G[1].a, g2 = h ? G[2].b : G[2].a;
+        s[h] = fma2(g2, g2, fma2(g1, g1, mul2(g0, g0)));
+        a[h][0] = fma2(t, g0, h ? x[0].b : x[0].a);
+        a[h][1] = fma2(t, g1, h ? x[1].b : x[1].a);
+        a[h][2] = fma2(t, g2, h ? x[2].b : x[2].a);
+    }
+    const uint32_t key = min(min(min(below_key(a[0][0]), below_key(a[0][1])), min(below_key(a[0][2]), below_key(a[1][0]))),
+                             min(below_key(a[1][1]), below_key(a[1][2])));
+    const float most = fmaxf(fmaxf(s[0].x, s[0].y), fmaxf(s[1].x, s[1].y));
+    if (tau_in_range && most <= 0x1p40f && key >= (67u << 24) - 1u) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float2 mz;
+            const float2 l = root2_rn(f2(fmaxf(s[h].x, 0x1p-80f), fmaxf(s[h].y, 0x1p-80f)), mz);
+            const float2 md = fma2(f2(-tau), l, f2(-1.0f));  // -(1 + tau |G|)
+            const float2 r = rcp2_step(md, f2(rcp_1ulp(-md.x), rcp_1ulp(-md.y)));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) q[h][k] = quot2_rn(a[h][k], md, r);
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float dx = fmaf(tau, __fsqrt_rn(s[h].x), 1.0f), dy = fmaf(tau, __fsqrt_rn(s[h].y), 1.0f);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) q[h][k] = f2(__fdiv_rn(a[h][k].x, dx), __fdiv_rn(a[h][k].y, dy));
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float2 e0 = sub2(h ? x[0].b : x[0].a, q[h][0]), e1 = sub2(h ? x[1].b : x[1].a, q[h][1]),
+                     e2 = sub2(h ? x[2].b : x[2].a, q[h][2]);
+        d[h] = fma2(e2, e2, fma2(e1, e1, mul2(e0, e0)));
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) x[k] = Quad{q[0][k], q[1][k]};
+    return Quad{d[0], d[1]};
+}
 
-// Thread assignments (8 x 128 tiles, 256 threads; fixed for the whole column march, so
-// that index arithmetic is done once per block):
-//  - update: thread t owns slice nn = t % 128 and rows 4h .. 4h+3 (h = t / 128), walking
-//    down the rows with the v value of the row below kept in a register;
-//  - divergence: the same slice, v rows 5h .. 5h+4 (of nine), xi_1 of the row above kept in
-//    a register; thread t < 9 also computes v at slice n0+128 of row t;
-//  - thread 0 issues the TMA loads.
-// Every wait on a load is bounded; a block whose wait gives up sets *err, drains its loads in
-// flight (bounded) and stops.
-template <int TR, int TN>
-__global__ void __launch_bounds__(kTvThreads, 3)
+// rlam = RN(1 / lam); lam_in_range: 2^-20 <= |lam| <= 2^20; tau_in_range: 0 <= tau <= 1.  kVecG: g is 16-byte aligned.  Every
+// wait on a load is bounded; a block whose wait gives up sets *err, drains its loads in flight
+// (bounded) and stops.
+template <bool kVecG>
+__global__ void __launch_bounds__(kTvThreads, kTvBlocks)
     tv_tiled_kernel(Geometry g, const int4 *__restrict__ cols, int col_begin, int col_end,
                     const int4 *__restrict__ work, const __grid_constant__ CUtensorMap xi_map,
-                    const __grid_constant__ CUtensorMap d_map, const float *__restrict__ D, float *__restrict__ xi_out,
-                    float tau, float *dq, int *err)
+                    const float *__restrict__ gin, float *__restrict__ xi_out, float lam, float rlam, int lam_in_range,
+                    const int *__restrict__ unsafe, float tau, int tau_in_range, float *dq, int *err)
 {
-    static_assert(TR == 8 && TN == 128 && kTvThreads == 256, "thread assignments are for 8 x 128 tiles");
-    using T = TvTile<TR, TN>;
+    using T = TvTile;
     extern __shared__ __align__(128) uint8_t tv_raw[];
     // align to 128 bytes by pointer arithmetic on the shared array itself
     uint8_t *const base = tv_raw + ((128u - (smem_addr(tv_raw) & 127u)) & 127u);
     float *const smf = reinterpret_cast<float *>(base);
     uint64_t *const bar = reinterpret_cast<uint64_t *>(base + T::OFF_BAR);
-    volatile int *const abort = reinterpret_cast<volatile int *>(base + T::OFF_BAR + 3 * 8);
+    volatile int *const abort = reinterpret_cast<volatile int *>(base + T::OFF_BAR + T::SLOTS * 8);
     auto sx = [&](int sl) { return smf + sl * T::XI_SLOT; };
-    auto sv = [&](int sl) { return smf + 3 * T::XI_SLOT + sl * T::V_PLANE; };
-    const int t = threadIdx.x;
+    auto sv = [&](int sl) { return smf + T::SLOTS * T::XI_SLOT + sl * T::V_PLANE; };
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
     const int4 wk = work[blockIdx.x];
     const int r0 = wk.x, n0 = wk.y, ca = wk.z, cb = wk.w;
-    const int64_t nsw = g.nstride_w;
-    auto col_at = [&](int c) { return (c >= col_begin && c < col_end) ? cols[c] : make_int4(0, 0, 0, 0); };
+    const int row = r0 + w, nq = n0 + 4 * lane;
+    const bool rcp_lam = lam_in_range && __ldg(unsafe) == 0;
+    auto col_at = [&](int c) { return (c >= col_begin && c < col_end) ? __ldg(cols + c) : make_int4(0, 0, 0, 0); };
+    // bit j: slice nq + j is in the field, has a next slice.  Values of other slices are computed but
+    // reach no voxel: v at the first slice past the end is read only under fwd.
+    unsigned in = 0, fwd = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        in |= (nq + j < g.ns ? 1u : 0u) << j;
+        fwd |= (nq + j + 1 < g.ns ? 1u : 0u) << j;
+    }
+    // clears the elements without a next slice: in a tile that ends before the field does there are
+    // none, and with whole quads of slices only a last element can be one
+    const bool inner = n0 + T::TN < g.ns, quads = (g.ns & 3) == 0;
+    auto mask_fwd = [&](Quad &x) {
+        if (inner) return;
+        if (quads)
+            x.b.y = fwd & 8u ? x.b.y : 0.0f;
+        else
+            x = keep4(x, fwd);
+    };
 
     if (t == 0) {
-        for (int k = 0; k < 3; ++k) mbar_init(bar + k, 1);
+        for (int k = 0; k < T::SLOTS; ++k) mbar_init(bar + k, 1);
         *abort = 0;
         mbar_fence_init();
         tma_prefetch_desc(&xi_map);
-        tma_prefetch_desc(&d_map);
     }
     __syncthreads();
     uint32_t phase = 0, pending = 0;  // per slot: parity of the next wait, load in flight (thread 0's view)
-    // plane c's xi box (rows r0-1 .., slices n0-4 ..) into ring slot `slot`, and its box of the
-    // differences of g (rows r0 .., slices n0 ..) into L2; thread 0 only
-    auto issue = [&](int c, int slot) {
+    auto issue = [&](int c, int slot) {  // plane c's xi box; thread 0 only
         const int4 ci = col_at(c);
         mbar_arrive_expect_tx(bar + slot, T::BOX_BYTES);
         tma_load_3d(sx(slot), &xi_map, bar + slot, n0 - 4, ci.x - ci.y + r0 - 1, 0);
         pending |= 1u << slot;
-        if (c >= ca) tma_prefetch_l2_3d(&d_map, n0, ci.x - ci.y + r0, 0);
     };
-    auto wait_slot = [&](int slot) {  // warp-uniform
-        const bool ok = mbar_wait_warp(bar + slot, (phase >> slot) & 1u, abort);
-        if (ok) {
+    auto wait_slot = [&](int slot) {  // warp-uniform; a wait that gives up sets *abort
+        if (mbar_wait_warp(bar + slot, (phase >> slot) & 1u, abort)) {
             phase ^= 1u << slot;
             pending &= ~(1u << slot);
         }
-        return ok;
     };
-
-    const int nn = t & (TN - 1), h = t >> 7;
-    const int n = n0 + nn;
-    const bool nin = n < g.ns, nbk = n > 0, nfw = n + 1 < g.ns;
-    // v = div xi of the plane with entry ci (xi box X), previous plane cp (xi box Xp), next cn
+    // offset of the lane's first voxel on the plane with entry ci
+    auto offset = [&](int4 ci) { return ((int64_t)ci.x + (row - ci.y)) * g.nstride_w + nq; };
+    // the lane's g at offset o (0 where there is none) and its slice n0+128 (lane 31)
+    auto load_g = [&](bool there, int64_t o) {
+        if (w == T::TR || !there || in == 0u) return zero4();
+        const float *p = gin + o;
+        if constexpr (kVecG) return quad(__ldg(reinterpret_cast<const float4 *>(p)));
+        return Quad{f2(__ldg(p), __ldg(p + 1)), f2(__ldg(p + 2), __ldg(p + 3))};
+    };
+    const bool edge_lane = lane == 31 && nq + 4 < g.ns && w < T::TR;
+    auto load_edge = [&](bool there, int64_t o) { return edge_lane && there ? __ldg(gin + o + 4) : 0.0f; };
+    // v = div xi of the lane's voxels on the plane with entry ci (xi box X), previous plane cp (xi box
+    // Xp), next cn; stored to V (warp 8: also slice n0+128 of the tile's rows)
     auto divergence = [&](int4 ci, int4 cp, int4 cn, const float *X, const float *Xp, float *V) {
         const float *s0 = X, *s1 = X + T::XC, *s2 = X + 2 * T::XC, *s2p = Xp + 2 * T::XC;
-        float up = s1[(5 * h) * T::XS + nn + 4];  // xi_1 of the row above the first
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            const int rr = 5 * h + m;
-            if (rr >= T::VR) break;
-            const int row = r0 + rr, b = (rr + 1) * T::XS + nn + 4;
-            const float a0m = s0[b - 1], a0 = s0[b], a1 = s1[b], a2p = s2p[b], a2 = s2[b];
-            float d = 0.0f;
-            if (tv_row_in(ci, row) && nin) {
-                if (nbk) d -= a0m;
-                if (nfw) d += a0;
-                if (row > ci.y) d -= up;
-                if (row + 1 < ci.z) d += a1;
-                if (tv_row_in(cp, row)) d -= a2p;
-                if (tv_row_in(cn, row)) d += a2;
-            }
-            V[rr * T::GS + nn] = d;
-            up = a1;
+        Quad d = zero4();
+        if (tv_row_in(ci, row)) {  // warp-uniform, as all conditions on rows and columns
+            const int b = (w + 1) * T::XS + 4 * lane + 4;
+            Quad a0 = lds4(s0 + b);
+            float prev = __shfl_up_sync(0xffffffffu, a0.b.y, 1);
+            if (lane == 0) prev = n0 > 0 ? s0[b - 1] : 0.0f;
+            const Quad a0m{f2(prev, a0.a.x), f2(a0.a.y, a0.b.x)};
+            mask_fwd(a0);
+            d = add4(sub4(d, a0m), a0);
+            if (row > ci.y) d = sub4(d, lds4(s1 + b - T::XS));
+            if (row + 1 < ci.z) d = add4(d, lds4(s1 + b));
+            if (tv_row_in(cp, row)) d = sub4(d, lds4(s2p + b));
+            if (tv_row_in(cn, row)) d = add4(d, lds4(s2 + b));
         }
-        if (t < T::VR) {  // slice n0+TN of row t
-            const int rr = t, row = r0 + rr, ne = n0 + TN, b = (rr + 1) * T::XS + TN + 4;
-            float d = 0.0f;
-            if (tv_row_in(ci, row) && ne < g.ns) {
-                d -= s0[b - 1];
-                if (ne + 1 < g.ns) d += s0[b];
-                if (row > ci.y) d -= s1[b - T::XS];
-                if (row + 1 < ci.z) d += s1[b];
-                if (tv_row_in(cp, row)) d -= s2p[b];
-                if (tv_row_in(cn, row)) d += s2[b];
+        *reinterpret_cast<float4 *>(V + w * T::VS + 4 * lane) = make_float4(d.a.x, d.a.y, d.b.x, d.b.y);
+        if (w == T::TR && lane < T::TR) {  // slice n0+TN of row r0 + lane
+            const int rw = r0 + lane, ne = n0 + T::TN, b = (lane + 1) * T::XS + T::TN + 4;
+            float e = 0.0f;
+            if (tv_row_in(ci, rw) && ne < g.ns) {
+                e -= s0[b - 1];
+                if (ne + 1 < g.ns) e += s0[b];
+                if (rw > ci.y) e -= s1[b - T::XS];
+                if (rw + 1 < ci.z) e += s1[b];
+                if (tv_row_in(cp, rw)) e -= s2p[b];
+                if (tv_row_in(cn, rw)) e += s2[b];
             }
-            V[rr * T::GS + TN] = d;
+            V[lane * T::VS + T::TN] = e;
         }
+        return d;
     };
 
-    // planes ca-1, ca, ca+1 into slots 0, 1, 2 (plane c sits in slot (c - ca + 1) mod 3)
+    // planes ca-1, ca, ca+1 into slots 0, 1, 2 (plane c sits in slot (c - ca + 1) mod 3; plane c+2 is
+    // issued when plane c-1 is done with)
     if (t == 0)
-        for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < T::SLOTS; ++k)
             if (ca - 1 + k <= cb) issue(ca - 1 + k, k);
+    int4 ci = col_at(ca), cn = col_at(ca + 1);
+    int64_t oc = offset(ci), on = offset(cn);
+    Quad gc = load_g(tv_row_in(ci, row), oc), gn = load_g(tv_row_in(cn, row), on);
+    Quad gd = load_g(tv_row_in(ci, row + 1), oc + g.nstride_w);
+    float ge = load_edge(tv_row_in(ci, row), oc), gne = load_edge(tv_row_in(cn, row), on);
     wait_slot(0);
     wait_slot(1);
+    Quad v = divergence(ci, col_at(ca - 1), cn, sx(1), sx(0), sv(0));
     __syncthreads();
-    if (!*abort) divergence(col_at(ca), col_at(ca - 1), col_at(ca + 1), sx(1), sx(0), sv(0));
-    __syncthreads();
+    if (t == 0 && ca + 2 <= cb) issue(ca + 2, 0);
     float dmax = 0.0f;
-    int sp = 0, sc = 1, sn = 2;  // slots of planes c-1, c, c+1
-    int vc = 0;                  // v slot of plane c
-    const int64_t rowoff = (int64_t)(r0 + 4 * h) * nsw + n;
+    int sc = 1, sn = 2;  // slots of planes c, c+1
+    int vc = 0;          // v slot of plane c
 #pragma unroll 1
     for (int c = ca; c < cb; ++c) {
-        const int4 ci = col_at(c), cn = col_at(c + 1);
-        const int64_t o0 = (int64_t)(ci.x - ci.y) * nsw + rowoff;
-        // this plane's differences of g, in flight during the wait and the divergence
-        float dg[4][3];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const bool in = tv_row_in(ci, r0 + 4 * h + m) && nin;
-            const int64_t o = o0 + m * nsw;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) dg[m][k] = in ? __ldg(D + k * g.plane_w + o) : 0.0f;
-        }
+        const int4 c2 = col_at(c + 2);
+        // g of the next two planes, in flight during this one
+        const int64_t o2 = offset(c2);
+        const bool there2 = c + 2 <= cb && tv_row_in(c2, row);
+        const Quad g2 = load_g(there2, o2), gd1 = load_g(tv_row_in(cn, row + 1), on + g.nstride_w);
+        const float g2e = load_edge(there2, o2);
         wait_slot(sn);  // plane c+1
-        // past this barrier every thread is done with iteration c-1: the slot of plane c-1 and
-        // the v slot of plane c-1 are free
-        __syncthreads();
-        if (*abort) break;
-        if (t == 0 && c + 2 <= cb) issue(c + 2, sp);
-        divergence(cn, ci, col_at(c + 2), sx(sn), sx(sc), sv(vc ^ 1));
-        __syncthreads();
-        const float *Vc = sv(vc), *Vn = sv(vc ^ 1);
-        const float *x0 = sx(sc), *x1 = x0 + T::XC, *x2 = x0 + 2 * T::XC;
-        float v0 = Vc[(4 * h) * T::GS + nn];
+        const Quad vn = divergence(cn, ci, c2, sx(sn), sx(sc), sv(vc ^ 1));
+        // the next slice's v and g
+        float vr = __shfl_down_sync(0xffffffffu, v.a.x, 1), gr = __shfl_down_sync(0xffffffffu, gc.a.x, 1);
+        if (w < T::TR && tv_row_in(ci, row) && in != 0u) {
+            const float *Vc = sv(vc) + w * T::VS;
+            const float *x0 = sx(sc) + (w + 1) * T::XS + 4 * lane + 4;
+            Quad x[3] = {lds4(x0), lds4(x0 + T::XC), lds4(x0 + 2 * T::XC)};
+            if (lane == 31) vr = Vc[T::TN], gr = ge;
+            Quad G[3] = {sub4(sub4(Quad{f2(v.a.y, v.b.x), f2(v.b.y, vr)}, v),
+                              div4_rn(sub4(Quad{f2(gc.a.y, gc.b.x), f2(gc.b.y, gr)}, gc), lam, rlam, rcp_lam)),
+                         zero4(), zero4()};
+            mask_fwd(G[0]);
+            if (row + 1 < ci.z)
+                G[1] = sub4(sub4(lds4(Vc + T::VS + 4 * lane), v), div4_rn(sub4(gd, gc), lam, rlam, rcp_lam));
+            if (tv_row_in(cn, row)) G[2] = sub4(sub4(vn, v), div4_rn(sub4(gn, gc), lam, rlam, rcp_lam));
+            const Quad d = tv_step(x, G, tau, tau_in_range != 0);
+            float *o = xi_out + oc;
+            if (in == 0xfu) {
+                dmax = fmaxf(fmaxf(dmax, fmaxf(d.a.x, d.a.y)), fmaxf(d.b.x, d.b.y));
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int rr = 4 * h + m, row = r0 + rr;
-            const int a = rr * T::GS + nn, b = (rr + 1) * T::XS + nn + 4;
-            const float vr = Vc[a + 1], vd = Vc[a + T::GS];
-            if (tv_row_in(ci, row) && nin) {
-                float g1 = 0.0f, g2 = 0.0f, g3 = 0.0f;
-                if (nfw) g1 = (vr - v0) - dg[m][0];
-                if (row + 1 < ci.z) g2 = (vd - v0) - dg[m][1];
-                if (tv_row_in(cn, row)) g3 = (Vn[a] - v0) - dg[m][2];
-                float s = g1 * g1;
-                s = fmaf(g2, g2, s);
-                s = fmaf(g3, g3, s);
-                const float denom = fmaf(tau, __fsqrt_rn(s), 1.0f);
-                const float xa = x0[b], xb = x1[b], xc = x2[b];
-                const float q1 = __fdiv_rn(fmaf(tau, g1, xa), denom);
-                const float q2 = __fdiv_rn(fmaf(tau, g2, xb), denom);
-                const float q3 = __fdiv_rn(fmaf(tau, g3, xc), denom);
-                const float e1 = xa - q1, e2 = xb - q2, e3 = xc - q3;
-                float d = e1 * e1;
-                d = fmaf(e2, e2, d);
-                d = fmaf(e3, e3, d);
-                dmax = fmaxf(dmax, d);
-                const int64_t o = o0 + m * nsw;
-                xi_out[o] = q1;
-                xi_out[g.plane_w + o] = q2;
-                xi_out[2 * g.plane_w + o] = q3;
+                for (int k = 0; k < 3; ++k)
+                    *reinterpret_cast<float4 *>(o + k * g.plane_w) = make_float4(x[k].a.x, x[k].a.y, x[k].b.x, x[k].b.y);
+            } else {
+                const float dd[4] = {d.a.x, d.a.y, d.b.x, d.b.y};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if ((in >> j) & 1u) {
+                        dmax = fmaxf(dmax, dd[j]);
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            const float2 h = j < 2 ? x[k].a : x[k].b;
+                            o[k * g.plane_w + j] = j & 1 ? h.y : h.x;
+                        }
+                    }
             }
-            v0 = vd;
         }
-        const int tmp = sp;
-        sp = sc;
+        // past this barrier every warp is done with plane c's xi slot and v slot
+        __syncthreads();
+        if (__shfl_sync(0xffffffffu, *abort, 0)) break;
+        if (t == 0 && c + 3 <= cb) issue(c + 3, sc);
+        v = vn;
+        gc = gn, ge = gne, gn = g2, gne = g2e, gd = gd1;
+        ci = cn, cn = c2;
+        oc = on, on = o2;
+        const int s_free = sc;
         sc = sn;
-        sn = tmp;
+        sn = 3 - s_free - sn;
         vc ^= 1;
     }
     if (t == 0 && *abort) {
         // loads still in flight must land before the block's shared memory goes away
-        for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < T::SLOTS; ++k)
             if ((pending >> k) & 1u) mbar_wait_bounded(bar + k, (phase >> k) & 1u, kDrainTries);
         atomicExch(err, 1);
     }

@@ -1157,39 +1157,44 @@ int context_init(int device, void *stream, bool use_stream, potts_context **out)
 #include "shard.cuh"
 
 // Work items, shared-memory size and the tensor maps of the two xi buffers (3 planes each,
-// boxes of XS slices x XR lines x 3 components) of the tiled TV kernel for TR x TN tiles.
-template <int TR, int TN>
-int tv_tiled_setup(potts_context *ctx, const Geometry &g, const float *xi_a, const float *xi_b, const float *D,
-                   CUtensorMap *maps)
+// boxes of XS slices x XR lines x 3 components) of the tiled TV kernel.
+int tv_tiled_setup(potts_context *ctx, const Geometry &g, const float *xi_a, const float *xi_b, CUtensorMap *maps)
 {
-    using T = potts::TvTile<TR, TN>;
-    POTTS_TRY(plan_tiles(ctx, g.ns, TileChoice{TR, TN, 1, 64}));
-    POTTS_CUDA(cudaFuncSetAttribute(potts::tv_tiled_kernel<TR, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    using T = potts::TvTile;
+    const potts_mapping &m = ctx->mapping.m;
+    int segment = 64;
+    march_time({{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, T::TR, T::TN, potts::kTvBlocks * std::max(ctx->n_sm, 1), 0,
+               &segment);
+    POTTS_TRY(plan_tiles(ctx, g.ns, TileChoice{T::TR, T::TN, 4, segment}));
+    POTTS_CUDA(cudaFuncSetAttribute(potts::tv_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    T::SMEM_BYTES));
+    POTTS_CUDA(cudaFuncSetAttribute(potts::tv_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     T::SMEM_BYTES));
     const uint64_t dims[3] = {(uint64_t)g.nstride_w, (uint64_t)g.n_lines, 3};
     const uint64_t strides[2] = {sizeof(float) * (uint64_t)g.nstride_w, sizeof(float) * (uint64_t)g.plane_w};
     const uint32_t box[3] = {(uint32_t)T::XS, (uint32_t)T::XR, 3};
     POTTS_TRY(encode_map(&maps[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, xi_a, 3, dims, strides, box));
     POTTS_TRY(encode_map(&maps[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, xi_b, 3, dims, strides, box));
-    const uint32_t dbox[3] = {(uint32_t)TN, (uint32_t)TR, 3};  // differences of g: L2 prefetch boxes
-    POTTS_TRY(encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, D, 3, dims, strides, dbox));
     return POTTS_OK;
 }
 
-template <int TR, int TN>
-void tv_tiled_launch(potts_context *ctx, const Geometry &g, const CUtensorMap &xi_map, const CUtensorMap &d_map,
-                     const float *D, float *xi_out, float tau, float *dq)
+void tv_tiled_launch(potts_context *ctx, const Geometry &g, const CUtensorMap &xi_map, const float *d_g, float *xi_out,
+                     float lam, float tau, float *dq)
 {
     if (ctx->n_work == 0) return;
     const MappingCopy &mc = ctx->mapping;
-    potts::tv_tiled_kernel<TR, TN><<<ctx->n_work, potts::kTvThreads, potts::TvTile<TR, TN>::SMEM_BYTES, ctx->stream>>>(
+    const bool in_range = std::fabs(lam) >= 0x1p-20f && std::fabs(lam) <= 0x1p20f;
+    int *err = (int *)ctx->err.p;
+    auto kern = reinterpret_cast<uintptr_t>(d_g) % 16 == 0 ? potts::tv_tiled_kernel<true> : potts::tv_tiled_kernel<false>;
+    kern<<<ctx->n_work, potts::kTvThreads, potts::TvTile::SMEM_BYTES, ctx->stream>>>(
         g, static_cast<const int4 *>(ctx->cols.p), (int)mc.m.col_begin, (int)mc.m.col_end,
-        static_cast<const int4 *>(ctx->work.p), xi_map, d_map, D, xi_out, tau, dq, (int *)ctx->err.p);
+        static_cast<const int4 *>(ctx->work.p), xi_map, d_g, xi_out, lam, 1.0f / lam, in_range ? 1 : 0, err + 1, tau,
+        tau >= 0.0f && tau <= 1.0f ? 1 : 0, dq, err);
 }
 
 // TV-L2 denoising (chambolle(), totalvarmin/chambolle.cpp:220-276) of d_g in
-// place; xi (two halves of 3 planes for the fused forms), v (split form) and the
-// differences of g (tiled form) live in the context's state buffer, laid out like g.
+// place; xi (two halves of 3 planes for the fused forms) and v (split form) live in
+// the context's state buffer, laid out like g.
 int tv_run(potts_context *ctx, float *d_g, float lam, float tau, int iters, int variant, potts_stats *stats)
 {
     const MappingCopy &mc = ctx->mapping;
@@ -1204,14 +1209,13 @@ int tv_run(potts_context *ctx, float *d_g, float lam, float tau, int iters, int 
     cudaStream_t s = ctx->stream;
     // the tiled kernel's TMA boxes need 16-byte line strides, else the per-voxel fused kernel runs
     const bool tiled = variant == POTTS_VARIANT_FUSED && mc.m.nstride % 4 == 0;
-    // split: xi, v; fused forms: xi ping-pong; tiled: and the three difference planes of g
-    const size_t planes = variant == POTTS_VARIANT_PLAIN ? 4 : tiled ? 9 : 6;
+    // split: xi, v; fused forms: xi ping-pong
+    const size_t planes = variant == POTTS_VARIANT_PLAIN ? 4 : 6;
     POTTS_TRY(ensure(ctx, ctx->state, sizeof(float) * planes * (size_t)std::max<int64_t>(g.plane_w, 1)));
     POTTS_TRY(ensure(ctx, ctx->dq, sizeof(float) * (size_t)std::max(iters, 1)));
-    POTTS_TRY(ensure(ctx, ctx->err, sizeof(int)));
+    POTTS_TRY(ensure(ctx, ctx->err, 2 * sizeof(int)));  // error word, tv_range_kernel's flag
     float *xi = static_cast<float *>(ctx->state.p), *v = xi + 3 * g.plane_w;
     float *xi_b = xi + 3 * g.plane_w;  // fused forms: the second half
-    float *dgp = xi + 6 * g.plane_w;    // tiled form: differences of g
     float *dq = static_cast<float *>(ctx->dq.p);
     ctx->seg_used = 0;
     ctx->seg_open = false;
@@ -1220,22 +1224,21 @@ int tv_run(potts_context *ctx, float *d_g, float lam, float tau, int iters, int 
     // xi starts at zero; every other plane is written at the voxels it is read at before it is read
     POTTS_CUDA(cudaMemsetAsync(ctx->state.p, 0, sizeof(float) * 3 * (size_t)std::max<int64_t>(g.plane_w, 1), s));
     POTTS_CUDA(cudaMemsetAsync(dq, 0, sizeof(float) * (size_t)std::max(iters, 1), s));
-    POTTS_CUDA(cudaMemsetAsync(ctx->err.p, 0, sizeof(int), s));
+    POTTS_CUDA(cudaMemsetAsync(ctx->err.p, 0, 2 * sizeof(int), s));
     const unsigned nb = plain_blocks(g, 0, g.ns);
     // tiled form: the Potts kernel's column table and work items for 8 x 128 tiles
-    constexpr int kTvRows = 8, kTvSlices = 128;
-    CUtensorMap xi_maps[3];  // of xi, xi_b and the differences of g
+    CUtensorMap xi_maps[2];  // of xi and xi_b
     int map_in = 0;          // the map of the buffer the next launch reads
     if (tiled && g.n_lines > 0 && iters > 0) {
-        POTTS_TRY((tv_tiled_setup<kTvRows, kTvSlices>(ctx, g, xi, xi_b, dgp, xi_maps)));
-        potts::tv_gdiff_kernel<<<nb, potts::kPlainThreads, 0, s>>>(g, d_g, dgp, lam);
+        POTTS_TRY(tv_tiled_setup(ctx, g, xi, xi_b, xi_maps));
+        potts::tv_range_kernel<<<nb, potts::kPlainThreads, 0, s>>>(g, d_g, (int *)ctx->err.p + 1);
         ctx->total_launches += 1;
     }
     if (g.n_lines > 0) {
         POTTS_TRY(seg_begin(ctx));
         for (int it = 0; it < iters; ++it) {
             if (tiled) {
-                tv_tiled_launch<kTvRows, kTvSlices>(ctx, g, xi_maps[map_in], xi_maps[2], dgp, xi_b, tau, dq + it);
+                tv_tiled_launch(ctx, g, xi_maps[map_in], d_g, xi_b, lam, tau, dq + it);
                 std::swap(xi, xi_b);
                 map_in ^= 1;
                 ctx->loop_launches += 1;

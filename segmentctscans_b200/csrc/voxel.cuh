@@ -32,8 +32,8 @@ __device__ __forceinline__ float fmax_ref(float a, float b) { return (a < b) ? b
 // documented error of rsqrt):
 //   l = RN(sqrt(s))  one Goldschmidt step for sqrt(s) and 1 / (2 sqrt(s)) and a
 //                    correction by the remainder s - g^2;
-//   r = RN(1 / l)    a Newton step from 2 h, but for a few mantissas (its remainder is
-//                    enlarged by an ulp: for the largest mantissa the step ends on a tie);
+//   r = RN(1 / l)    a step from 2 h with the remainder f and 2 f^2 (a Newton step's f alone
+//                    ends on a tie for the largest mantissa), but for a few mantissas;
 //   RN(a / l)        q = RN(a r) is within two ulp, one correction by the
 //                    remainder brings it within one, and the second then gives
 //                    the correctly rounded quotient (P. W. Markstein, IBM J.
@@ -73,7 +73,7 @@ __device__ __forceinline__ void shrink_rn(float h0, float h1, float h2, float s,
     const float l = fmaf(fmaf(-g, g, s), h, g);
     const float t = h + h;
     const float f = fmaf(-l, t, 1.0f);
-    const float r = fmaf(f * 0x1.000002p0f, t, t);
+    const float r = fmaf(fmaf(f + f, f, f), t, t);
     const float lm1 = l - 1.0f;
     const float a0 = lm1 * h0, a1 = lm1 * h1, a2 = lm1 * h2;
     if (s <= 0x1p40f && none_below_2m60(a0, a1, a2)) {
@@ -504,6 +504,32 @@ __device__ __forceinline__ unsigned dual_needs_loop_pair(const float2 (&q)[K][3]
     return (l0 ? 1u : 0u) | (l1 ? 2u : 0u);
 }
 
+// The steps of shrink_rn for two values, with the signs that save negations (two instructions for a
+// pair): RN(sqrt(s)) and mz ~ -1 / (2 sqrt(s)) for 2^-80 <= s <= 2^40; RN(1 / b) (but for a few
+// mantissas, see shrink_rn) from mb = -b and a reciprocal r0 of b within an ulp or so; RN(a / b) from
+// mb and rcp2_step's r.
+__device__ __forceinline__ float2 root2_rn(float2 s, float2 &mz)
+{
+    const float2 y = f2(rsqrt_2ulp(s.x), rsqrt_2ulp(s.y));
+    float2 g = mul2(s, y);
+    mz = mul2(f2(-0.5f), y);
+    const float2 e = fma2(g, mz, f2(0.5f));
+    g = fma2(g, e, g);
+    mz = fma2(mz, e, mz);
+    return fma2(fma2(g, g, neg2(s)), mz, g);
+}
+__device__ __forceinline__ float2 rcp2_step(float2 mb, float2 r0)
+{
+    const float2 f = fma2(mb, r0, f2(1.0f));
+    return fma2(fma2(add2(f, f), f, f), r0, r0);
+}
+__device__ __forceinline__ float2 quot2_rn(float2 a, float2 mb, float2 r)
+{
+    float2 q = mul2(a, r);
+    q = fma2(fma2(mb, q, a), r, q);
+    return fma2(fma2(mb, q, a), r, q);
+}
+
 // dykstra_sweep of two independent voxels (.x and .y) with the paired
 // instructions; max_dd receives the largest squared step of each.
 template <int K>
@@ -527,15 +553,9 @@ __device__ __forceinline__ void dykstra_sweep_pair(float2 (&q)[K][3], float2 (&P
             const bool x = s.x > thr.len_gt_one, y = s.y > thr.len_gt_one;
             if (x || y) {
                 const float2 s1 = f2(x ? s.x : 1.0f, y ? s.y : 1.0f);
-                const float2 rs = f2(rsqrt_2ulp(s1.x), rsqrt_2ulp(s1.y));  // shrink_rn
-                float2 g = mul2(s1, rs), z = mul2(f2(0.5f), rs);
-                const float2 e = fma2(neg2(g), z, f2(0.5f));
-                g = fma2(g, e, g);
-                z = fma2(z, e, z);
-                const float2 l = fma2(fma2(neg2(g), g, s1), z, g), ml = neg2(l);
-                const float2 t = add2(z, z);
-                const float2 f = fma2(ml, t, f2(1.0f));
-                const float2 r = fma2(mul2(f, f2(0x1.000002p0f)), t, t);
+                float2 mz;
+                const float2 l = root2_rn(s1, mz), ml = neg2(l);  // as in shrink_rn
+                const float2 r = rcp2_step(ml, mul2(f2(-2.0f), mz));
                 const float2 lm1 = add2(l, f2(-1.0f));
                 float2 m[3];
 #pragma unroll
@@ -543,11 +563,7 @@ __device__ __forceinline__ void dykstra_sweep_pair(float2 (&q)[K][3], float2 (&P
                 if (s.x <= 0x1p40f && s.y <= 0x1p40f && none_below_2m60(m[0].x, m[1].x, m[2].x) &&
                     none_below_2m60(m[0].y, m[1].y, m[2].y)) {
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        float2 v = mul2(m[a], r);
-                        v = fma2(fma2(ml, v, m[a]), r, v);
-                        n[a] = fma2(fma2(ml, v, m[a]), r, v);
-                    }
+                    for (int a = 0; a < 3; ++a) n[a] = quot2_rn(m[a], ml, r);
                 } else {
                     if (x) {
                         const float3 w = shrink_ops(h[0].x, h[1].x, h[2].x, s.x);

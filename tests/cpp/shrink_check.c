@@ -1,7 +1,7 @@
 /* The square root, reciprocal and quotients of csrc/voxel.cuh's shrink_rn against the IEEE
  * operations: l = RN(sqrt(s)) for every s in [1, 4) and every reciprocal square root within 2 ulp
  * (larger s are these times a power of four); r = RN(1 / l) but for the few l that are counted;
- * RN(a / l) by two corrections, for these l over every numerator of two binades, and for random
+ * the same step from a reciprocal of any b within 1 ulp; RN(a / l) by two corrections, for these l over every numerator of two binades, and for random
  * operands, ends of a binade among them, over the range 1 <= l <= 2^20, a zero or at least 2^-60.
  * Prints what differs (other than in the sign of a zero). */
 #include <math.h>
@@ -38,7 +38,7 @@ static void root(float s, float y, float *l, float *r)
     *l = fmaf(fmaf(-g, g, s), h, g);
     const float t = h + h;
     const float f = fmaf(-*l, t, 1.0f);
-    *r = fmaf(f * 0x1.000002p0f, t, t);
+    *r = fmaf(fmaf(f + f, f, f), t, t);
 }
 
 static long quotient(float a, float l, float r)
@@ -67,6 +67,18 @@ int main(int argc, char **argv)
             ++inexact;
             l_done = l, r_done = r;
             for (uint32_t m = 0x3f800000u; m < 0x40800000u && bad < 20; ++m) bad += quotient(bits(m), l, r);
+        }
+    }
+    /* the same step from a reciprocal within 1 ulp, for every divisor's mantissa */
+    for (uint32_t i = 0x3f800000u; i < 0x40000000u && bad < 20; ++i) {
+        const float b = bits(i);
+        for (int d = -1; d <= 1; ++d) {
+            const float t = bits(bits_of(1.0f / b) + (uint32_t)d);
+            const float f = fmaf(-b, t, 1.0f), r = fmaf(fmaf(f + f, f, f), t, t);
+            if (r == 1.0f / b || (b == l_done && r == r_done)) continue;
+            ++inexact;
+            l_done = b, r_done = r;
+            for (uint32_t m = 0x3f800000u; m < 0x40800000u && bad < 20; ++m) bad += quotient(bits(m), b, r);
         }
     }
     for (long i = 0; i < n && bad < 20; ++i) {
