@@ -64,7 +64,8 @@ int tape_iterate(potts_tape *t, const TapeState &s, int it)
 {
     potts_context *ctx = t->ctx;
     const unsigned nb = plain_blocks(t->g, 0, t->g.ns);
-    potts::dual_kernel<K, float><<<nb, potts::kPlainThreads, 0, ctx->stream>>>(t->g, s.xi, s.vb, t->tau2, ctx->thr);
+    potts::dual_kernel<K, float><<<potts::dual_blocks<float>(nb), potts::kPlainThreads, 0, ctx->stream>>>(
+        t->g, s.xi, s.vb, t->tau2, ctx->thr);
     potts::primal_kernel<K, float><<<nb, potts::kPlainThreads, 0, ctx->stream>>>(t->g, s.xi, s.v, s.vb, t->d_u,
                                                                                  tape_params<K>(t), nullptr, it);
     ctx->total_launches += 2;
@@ -149,7 +150,7 @@ int tape_backward(potts_tape *t, float *d_grad_u, double *grad_ci, double *grad_
                 t->g, sk.v, sk1.xi, t->d_u, pp, t->tau2, static_cast<float *>(t->A.p),
                 static_cast<const float *>(t->P.p), static_cast<float *>(t->Q.p), d_grad_u,
                 static_cast<double *>(t->grads.p));
-            potts::adj_dual_kernel<K><<<nb, potts::kPlainThreads, 0, s>>>(
+            potts::adj_dual_kernel<K><<<potts::dual_blocks<float>(nb), potts::kPlainThreads, 0, s>>>(
                 t->g, sk.xi, sk.vb, t->tau1, t->tau2, ctx->thr, static_cast<float *>(t->X.p),
                 static_cast<const float *>(t->Q.p), static_cast<float *>(t->P.p));
             ctx->total_launches += 2;

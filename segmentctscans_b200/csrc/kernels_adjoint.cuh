@@ -65,11 +65,7 @@ __device__ void dykstra_vjp(const float (&p)[K][3], const float (&ybar)[K][3], f
                 sq = fmaf(h2, h2, sq);
                 float n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
                 if (sq > thr.len_gt_one) {
-                    const float l = __fsqrt_rn(sq);
-                    const float lm1 = l - 1.0f;
-                    n0 = __fdiv_rn(lm1 * h0, l);
-                    n1 = __fdiv_rn(lm1 * h1, l);
-                    n2 = __fdiv_rn(lm1 * h2, l);
+                    shrink_rn(h0, h1, h2, sq, n0, n1, n2);
                 }
                 const float d0 = 0.5f * (n0 - P[k][0]);
                 const float d1 = 0.5f * (n1 - P[k][1]);
@@ -299,60 +295,69 @@ __global__ void __launch_bounds__(kPlainThreads)
                     DykstraThresholds thr, float *__restrict__ X, const float *__restrict__ qbar,
                     float *__restrict__ pbar)
 {
-    const PlainIndex p = plain_index(g, 0, g.ns);
-    if (!p.valid) return;
-    const LineInfo li = load_line(g, p.line);
-    const int64_t o = p.line * g.nstride_w + p.n;
-    const bool hn = p.n + 1 < g.ns;
-    const bool hr = li.flags & kHasNextRow;
-    const bool hc = li.next_col >= 0;
-    const int64_t oc = hc ? (int64_t)li.next_col * g.nstride_w + p.n : o;
-    float vx[K - 1], vn[K - 1], vr[K - 1], vc[K - 1], x[3 * (K - 1)];
+    __shared__ LoopList<3 * K + 3 * (K - 1)> list;
+    if (threadIdx.x == 0) list.count = 0;
+    __syncthreads();
+    auto store = [&](int64_t o, const float (&pb)[K][3]) {
 #pragma unroll
-    for (int i = 0; i < K - 1; ++i) {
-        const float *b = vb + i * g.plane_w;
-        vx[i] = b[o];
-        vn[i] = hn ? b[o + 1] : 0.0f;
-        vr[i] = hr ? b[o + g.nstride_w] : 0.0f;
-        vc[i] = hc ? b[oc] : 0.0f;
-    }
+        for (int i = 0; i < K - 1; ++i)
 #pragma unroll
-    for (int j = 0; j < 3 * (K - 1); ++j) x[j] = xi[j * g.plane_w + o];
-    float pq[K][3];
-    dual_build_q<K>(pq, x, vx, vn, vr, vc, hn, hr, hc, tau2);
-    // Xtot = X + tau1 E^T (-grad+ qbar): (div^T qbar)_a(x) = h_a (qbar(x) - qbar(x + e_a))
-    float dt[K][3];
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-        const float *qb = qbar + i * g.plane_w;
-        const float q0 = qb[o];
-        dt[i][0] = hn ? q0 - qb[o + 1] : 0.0f;
-        dt[i][1] = hr ? q0 - qb[o + g.nstride_w] : 0.0f;
-        dt[i][2] = hc ? q0 - qb[oc] : 0.0f;
-    }
-    float yb[K][3];
-#pragma unroll
-    for (int i = 0; i < K - 1; ++i)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) yb[i][a] = X[(3 * i + a) * g.plane_w + o] + tau1 * (dt[i][a] - dt[K - 1][a]);
-    yb[K - 1][0] = yb[K - 1][1] = yb[K - 1][2] = 0.0f;
-    float pb[K][3];
-    if (dual_first_sweep_is_identity<K>(pq, thr)) {
+            for (int a = 0; a < 3; ++a) X[(3 * i + a) * g.plane_w + o] = pb[i][a] - pb[K - 1][a];
 #pragma unroll
         for (int i = 0; i < K; ++i)
 #pragma unroll
-            for (int a = 0; a < 3; ++a) pb[i][a] = yb[i][a];
-    } else {
-        dykstra_vjp<K>(pq, yb, pb, thr);
+            for (int a = 0; a < 3; ++a) pbar[(3 * i + a) * g.plane_w + o] = pb[i][a];
+    };
+#pragma unroll 1
+    for (int c = 0; c < kLoopChunks; ++c) {
+        const PlainIndex p = plain_index(g, 0, g.ns, (int64_t)blockIdx.x * kLoopChunks + c);
+        float pq[K][3], yb[K][3];
+        int64_t o = 0;
+        bool need = false;
+        if (p.valid) {
+            const DualPoint<K, float> d(g, xi, vb, p);
+            o = d.o;
+            dual_build_q<K>(pq, d.x, d.vx, d.vn, d.vr, d.vc, d.hn, d.hr, d.hc, tau2);
+            // Xtot = X + tau1 E^T (-grad+ qbar): (div^T qbar)_a(x) = h_a (qbar(x) - qbar(x + e_a))
+            const int64_t oc = d.hc ? (int64_t)load_line(g, p.line).next_col * g.nstride_w + p.n : o;
+            float dt[K][3];
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                const float *qb = qbar + i * g.plane_w;
+                const float q0 = qb[o];
+                dt[i][0] = d.hn ? q0 - qb[o + 1] : 0.0f;
+                dt[i][1] = d.hr ? q0 - qb[o + g.nstride_w] : 0.0f;
+                dt[i][2] = d.hc ? q0 - qb[oc] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < K - 1; ++i)
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    yb[i][a] = X[(3 * i + a) * g.plane_w + o] + tau1 * (dt[i][a] - dt[K - 1][a]);
+            yb[K - 1][0] = yb[K - 1][1] = yb[K - 1][2] = 0.0f;
+            need = !dual_first_sweep_is_identity<K>(pq, thr);
+            if (!need) store(o, yb);
+        }
+        // the voxels whose projection ran the loop, gathered as in dual_kernel
+        const int e = list.add(need);
+        if (need) {
+#pragma unroll
+            for (int j = 0; j < 3 * K; ++j) list.v[j][e] = pq[j / 3][j % 3];
+#pragma unroll
+            for (int j = 0; j < 3 * (K - 1); ++j) list.v[3 * K + j][e] = yb[j / 3][j % 3];
+            list.off[e] = o;
+        }
+        list.flush(c + 1 == kLoopChunks, [&](int i) {
+#pragma unroll
+            for (int j = 0; j < 3 * K; ++j) pq[j / 3][j % 3] = list.v[j][i];
+#pragma unroll
+            for (int j = 0; j < 3 * (K - 1); ++j) yb[j / 3][j % 3] = list.v[3 * K + j][i];
+            yb[K - 1][0] = yb[K - 1][1] = yb[K - 1][2] = 0.0f;
+            float pb[K][3];
+            dykstra_vjp<K>(pq, yb, pb, thr);
+            store(list.off[i], pb);
+        });
     }
-#pragma unroll
-    for (int i = 0; i < K - 1; ++i)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) X[(3 * i + a) * g.plane_w + o] = pb[i][a] - pb[K - 1][a];
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) pbar[(3 * i + a) * g.plane_w + o] = pb[i][a];
 }
 
 }  // namespace potts

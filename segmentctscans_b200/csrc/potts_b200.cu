@@ -817,11 +817,12 @@ void launch_dual(bool fast, unsigned nb, cudaStream_t s, const Geometry &g, ST *
 {
     if constexpr (!std::is_same_v<ST, double>) {
         if (fast) {
-            potts::dual_kernel<K, ST, true><<<nb, potts::kPlainThreads, 0, s>>>(g, xi, vb, tau2, thr);
+            potts::dual_kernel<K, ST, true><<<potts::dual_blocks<ST>(nb), potts::kPlainThreads, 0, s>>>(g, xi, vb, tau2,
+                                                                                                       thr);
             return;
         }
     }
-    potts::dual_kernel<K, ST, false><<<nb, potts::kPlainThreads, 0, s>>>(g, xi, vb, tau2, thr);
+    potts::dual_kernel<K, ST, false><<<potts::dual_blocks<ST>(nb), potts::kPlainThreads, 0, s>>>(g, xi, vb, tau2, thr);
 }
 
 template <int K, typename ST>
