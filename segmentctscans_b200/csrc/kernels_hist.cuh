@@ -25,7 +25,7 @@ constexpr int kHistThreads = 256;
 // ---------------------------------------------------------------------------
 // Per block: min and max over the in-mask values (only those > 0 when kPositive), one warp per
 // line (lines blockIdx.x * 8 + warp, then every gridDim.x * 8); FLT_MAX / -FLT_MAX when the block
-// saw none.  kVec: 16-byte loads (lines of a multiple of 4 values and stride, aligned field).
+// saw none.  kVec: 16-byte loads (lines of a stride of a multiple of 4 values, aligned field).
 template <bool kPositive, bool kVec>
 __global__ void __launch_bounds__(kHistThreads) minmax_partial_kernel(Geometry g, const float *__restrict__ f,
                                                                       float2 *__restrict__ partial)
@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(kHistThreads) minmax_partial_kernel(Geometry g
                 see(v.z);
                 see(v.w);
             }
+            if (lane < (g.ns & 3)) see(__ldg(line + (g.ns & ~3) + lane));
         } else {
             for (int n = lane; n < g.ns; n += 32) see(__ldg(line + n));
         }
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(kHistThreads) minmax_pair_partial_kernel(Geome
                 see(x.z, y.z);
                 see(x.w, y.w);
             }
+            if (lane < (g.ns & 3)) see(__ldg(lu + (g.ns & ~3) + lane), __ldg(lv + (g.ns & ~3) + lane));
         } else {
             for (int n = lane; n < g.ns; n += 32) see(__ldg(lu + n), __ldg(lv + n));
         }
@@ -244,8 +246,9 @@ struct GmTile {
     static constexpr int SMEM_BYTES = OFF_BAR + SLOTS * 8 + 8 + 128;  // + abort flag, alignment slack
 };
 constexpr int kGmThreads = 256;
+constexpr int kGmBlocks = 4;  // per multiprocessor
 
-__global__ void __launch_bounds__(kGmThreads, 4)
+__global__ void __launch_bounds__(kGmThreads, kGmBlocks)
     grad_magn_tiled_kernel(Geometry g, const int4 *__restrict__ cols, int col_begin, int col_end,
                            const int4 *__restrict__ work, const __grid_constant__ CUtensorMap u_map,
                            float *__restrict__ v, int *err)
@@ -368,28 +371,27 @@ __device__ __forceinline__ int hist_bin(float x, float start, float end, int nb)
     return (int)r;
 }
 
-// hist_bin without its division where that cannot change the bin.  rinv = __frcp_rn(end - start),
-// the correctly rounded reciprocal.  For |t| <= 1 the product RN((x - start) rinv) differs from
-// the quotient t = RN((x - start) / (end - start)) by at most 1.5 ulp(1) (relative errors of
-// 2^-24 in rinv, in the product and in t), so y' = fma(nb, product, -0.5) differs from
-// hist_bin's fma(nb, t, -0.5) by less than nb 4.2e-7.  The bin is round(y) (halves away from
-// zero, then clamped), which can only differ between y and y' when y' lies within that distance
-// of a half-integer: then, and for a non-finite y', the division decides.  The bins are the same
-// as hist_bin's for every input (one division in about 2 nb 1e-6 of the cases).  Away from a
-// half-integer, round(y) is the nearer of floor(y) and floor(y) + 1, which the fraction
-// f = y - floor(y) (exact for every finite y) picks: f > 1/2 rounds up.
-__device__ __forceinline__ int hist_bin_r(float x, float start, float end, float rinv, int nb)
+// hist_bin of start <= x <= end without its division where that cannot change the bin.  rinv =
+// __frcp_rn(end - start), the correctly rounded reciprocal.  For |t| <= 1 the product
+// RN((x - start) rinv) differs from the quotient t = RN((x - start) / (end - start)) by at most 1.5
+// ulp(1) (relative errors of 2^-24 in rinv, in the product and in t), so y' = fma(nb, product, -0.5)
+// differs from hist_bin's y by less than nb 4.2e-7, and the bin, round(y) (halves away from zero, then
+// clamped), can only differ from the integer k nearest to y' when y' lies within that distance of a
+// half-integer.  k comes from adding 1.5 2^23, whose units are then the last place (|y'| < 2^22: y' lies
+// in [-0.5, nb - 0.5] up to rounding), and needs no clamp away from half-integers.  near = 1/2 - (nb
+// 1e-6 + 1e-6) is the largest |y' - k| (exact) that decides; beyond it (one value in about 2 nb 1e-6 of
+// them) and for a NaN or infinite y' (an empty or subnormal range) the division does, but for y' near -1/2
+// and nb - 1/2 (x at start or end, a field saturated there), whose candidates clamp to one bin.  Seven
+// instructions for most values: floor and fraction with a clamp took about twice that.
+__device__ __forceinline__ float hist_near(int nb) { return 0.5f - fmaf((float)nb, 1e-6f, 1e-6f); }
+__device__ __forceinline__ int hist_bin_r(float x, float start, float end, float rinv, float near, int nb)
 {
+    constexpr float kMagic = 12582912.0f;  // 1.5 2^23
     const float y = fmaf((float)nb, __fmul_rn(__fsub_rn(x, start), rinv), -0.5f);
-    const float fl = floorf(y);
-    const float f = __fsub_rn(y, fl);
-    if (fabsf(__fsub_rn(f, 0.5f)) > fmaf((float)nb, 1e-6f, 1e-6f)) {  // false for a NaN or infinite y
-        const float r = f > 0.5f ? __fadd_rn(fl, 1.0f) : fl;  // f > 1/2 only where |y| < 2^23: exact
-        return (int)fminf(fmaxf(r, 0.0f), (float)(nb - 1));     // r is finite here
-    }
-    // near a half-integer: the bin is floor(y) or floor(y) + 1, clamped, which are the same at
-    // both ends (x at start or end, e.g. a field saturated there)
-    if (f == f && (__fadd_rn(fl, 1.0f) <= 0.0f || fl >= (float)(nb - 1))) return fl >= 0.0f ? nb - 1 : 0;
+    const float m = __fadd_rn(y, kMagic);
+    if (fabsf(__fsub_rn(y, __fsub_rn(m, kMagic))) < near) return __float_as_int(m) - __float_as_int(kMagic);
+    if (y < 0.0f) return 0;
+    if (y > (float)(nb - 1) && y < (float)nb) return nb - 1;
     return hist_bin(x, start, end, nb);
 }
 
@@ -428,8 +430,8 @@ __device__ __forceinline__ void warp_count(uint32_t id, Add add)
 }
 
 // Eight values of one line for one lane of a warp that walks the line in steps of 256 values
-// (slices base .. base+255): with kVec two 16-byte loads (quads base/4 + lane and + 32; lines of
-// a multiple of 4 values and stride, 16-byte aligned field), else eight coalesced 4-byte loads
+// (slices base .. base+255): with kVec two 16-byte loads (quads base/4 + lane and + 32; lines of a
+// stride of a multiple of 4 values, 16-byte aligned field), else eight coalesced 4-byte loads
 // (slices base + lane + 32 j).  Bit j of the result: value j exists.  Several loads in flight
 // per lane keep enough bytes moving to cover the memory latency.
 template <bool kVec>
@@ -443,7 +445,8 @@ __device__ __forceinline__ unsigned load8(const float *__restrict__ line, int ns
             if (4 * q < ns) {
                 const float4 t = __ldg(reinterpret_cast<const float4 *>(line) + q);
                 x[4 * h] = t.x, x[4 * h + 1] = t.y, x[4 * h + 2] = t.z, x[4 * h + 3] = t.w;
-                valid |= 0xfu << (4 * h);
+                const int left = ns - 4 * q;  // the last quad may reach into the line's padding
+                valid |= (left >= 4 ? 0xfu : (1u << left) - 1u) << (4 * h);
             }
         }
     } else {
@@ -472,19 +475,21 @@ __device__ __forceinline__ int slice8(int base, int lane, int j)
 // 1-D histogram (calc_hist.cpp:23-80) into shared-memory copies, flushed with one global atomic
 // per non-zero bin.  `copies` = 1 (one copy per block) or kHistThreads / 32 (one per warp: when a
 // few bins hold most voxels, warps then never contend for the same counter); copies * nb * 4
-// bytes of dynamic shared memory.
+// bytes of dynamic shared memory.  range: [rs, re] in device memory, or null.
 template <bool kJitter, bool kVec>
 __global__ void __launch_bounds__(kHistThreads) hist1d_kernel(Geometry g, const float *__restrict__ f, float rs,
-                                                              float re, int nb, int copies, float delta,
-                                                              uint64_t seed, uint32_t *__restrict__ ghist)
+                                                              float re, const float *__restrict__ range, int nb,
+                                                              int copies, float delta, uint64_t seed,
+                                                              uint32_t *__restrict__ ghist)
 {
     extern __shared__ uint32_t sh_all[];
+    if (range) rs = range[0], re = range[1];
     for (int i = threadIdx.x; i < nb * copies; i += blockDim.x) sh_all[i] = 0u;
     __syncthreads();
     uint32_t *sh_hist = sh_all + (copies > 1 ? (int)(threadIdx.x >> 5) * nb : 0);
     const float hd = delta * 0.5f;  // delta / 2, exact
     const float lo = rs - hd;
-    const float rinv = __frcp_rn(__fsub_rn(re, rs));
+    const float rinv = __frcp_rn(__fsub_rn(re, rs)), near = hist_near(nb);
     const int lane = threadIdx.x & 31;
     constexpr int kWarps = kHistThreads / 32;
     // one warp per line
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(kHistThreads) hist1d_kernel(Geometry g, const 
                         xv = __fadd_rn(xv, hist_jitter(seed, (uint64_t)L * g.ns + slice8<kVec>(base, lane, j), delta));
                     // x + 0 compares as x: without jitter the upper test needs no addition
                     if (lo <= xv && (kJitter ? __fadd_rn(xv, hd) : xv) <= re)
-                        id = (uint32_t)hist_bin_r(xv, rs, re, rinv, nb);
+                        id = (uint32_t)hist_bin_r(kJitter ? fmaxf(xv, rs) : xv, rs, re, rinv, near, nb);  // below rs: bin 0
                 }
                 // each lane adds its own 1 to its warp's copy (or the block's): grouping the lanes
                 // of one bin measured slower even where half the field sits in one bin
@@ -521,9 +526,12 @@ __global__ void __launch_bounds__(kHistThreads) hist1d_kernel(Geometry g, const 
 // The same with global atomics only (bin counts too large for shared memory).
 template <bool kJitter>
 __global__ void __launch_bounds__(kHistThreads) hist1d_global_kernel(Geometry g, const float *__restrict__ f,
-                                                                     float rs, float re, int nb, float delta,
-                                                                     uint64_t seed, uint32_t *__restrict__ ghist)
+                                                                     float rs, float re,
+                                                                     const float *__restrict__ range, int nb,
+                                                                     float delta, uint64_t seed,
+                                                                     uint32_t *__restrict__ ghist)
 {
+    if (range) rs = range[0], re = range[1];
     const float hd = delta * 0.5f;
     const float lo = rs - hd;
     for (int64_t L = blockIdx.x; L < g.n_lines; L += gridDim.x) {
@@ -543,9 +551,16 @@ __global__ void __launch_bounds__(kHistThreads) hist1d_global_kernel(Geometry g,
 
 // Ranges and layout of the 2-D histogram (uv-hist-kernel.cpp:133-150): the pair (x = u, y = grad
 // magnitude) counts at ybin * stride + xbin when it lies in [u_start, u_end] x [v_start, v_end].
+// dev: the four ends in device memory (us, ue, vs, ve), or null.
 struct UvRange {
     float us, ue, vs, ve;
     int nb, stride;
+    const float *dev;
+
+    __device__ __forceinline__ void load()
+    {
+        if (dev) us = dev[0], ue = dev[1], vs = dev[2], ve = dev[3];
+    }
 };
 
 // Both bins of the pair, or false outside the ranges.  ru / rv: __frcp_rn(ue - us) and
@@ -553,19 +568,20 @@ struct UvRange {
 __device__ __forceinline__ bool uv_bins(float x, float y, const UvRange &r, float ru, float rv, int &xb, int &yb)
 {
     if (!(r.us <= x && x <= r.ue && r.vs <= y && y <= r.ve)) return false;
-    xb = hist_bin_r(x, r.us, r.ue, ru, r.nb);
-    yb = hist_bin_r(y, r.vs, r.ve, rv, r.nb);
+    const float near = hist_near(r.nb);
+    xb = hist_bin_r(x, r.us, r.ue, ru, near, r.nb);
+    yb = hist_bin_r(y, r.vs, r.ve, rv, near, r.nb);
     return true;
 }
 
 // The 2-D histogram with its densest bins in every block's own shared memory.  The bins are
 // grouped into coarse cells of 2^cs x 2^cs bins (cdim cells per axis, at most kUvCoarseMax);
-// uv_coarse_kernel counts the cells over a sample of the lines, the host gives the densest
+// uv_coarse_kernel counts the cells over a sample of the lines, uv_select_kernel gives the densest
 // cells (up to kUvHotBins bins) a slot, and uv_hist_hot_kernel counts a voxel in its block's
 // slot counters when its cell has one, else with a global atomic.  Counts are exact either
 // way; the choice of cells only changes speed.
 constexpr int kUvCoarseMax = 64;    // coarse cells per axis
-constexpr int kUvHotBins = 32768;   // bins counted in a block's shared memory (128 KB)
+constexpr int kUvHotBins = 49152;   // bins counted in a block's shared memory (192 KB; 128 KB: 1.07 ms, 1.04)
 constexpr int kUvThreads = 1024;    // one block per multiprocessor: as many warps as it holds
 
 template <bool kVec>
@@ -574,6 +590,7 @@ __global__ void __launch_bounds__(kHistThreads) uv_coarse_kernel(Geometry g, con
                                                                  int cdim, int step, uint32_t *__restrict__ gcoarse)
 {
     __shared__ uint32_t sh[kUvCoarseMax * kUvCoarseMax];
+    r.load();
     const int cells = cdim * cdim;
     for (int i = threadIdx.x; i < cells; i += blockDim.x) sh[i] = 0u;
     __syncthreads();
@@ -601,6 +618,48 @@ __global__ void __launch_bounds__(kHistThreads) uv_coarse_kernel(Geometry g, con
         if (sh[i]) atomicAdd(gcoarse + i, sh[i]);
 }
 
+// Gives n_slots of the cells with the largest counts a slot: table[cell] = slot or -1,
+// slot_cell[slot] = cell.  The smallest count that gets one is found by bisection, then the cells
+// above it take slots, and those at it as many as are left (which of them does not matter).  One
+// block, a few microseconds; sorting the counts on the host took two copies, a wait and 0.2 ms.
+__global__ void __launch_bounds__(1024) uv_select_kernel(const uint32_t *__restrict__ counts, int cells, int n_slots,
+                                                         int16_t *__restrict__ table, int16_t *__restrict__ slot_cell)
+{
+    constexpr int kPer = kUvCoarseMax * kUvCoarseMax / 1024;
+    __shared__ int used;
+    uint32_t c[kPer];
+    bool in[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int i = (int)threadIdx.x + 1024 * k;
+        in[k] = i < cells;
+        c[k] = in[k] ? counts[i] : 0u;
+    }
+    uint32_t floor = 0;  // the largest count that at least n_slots cells reach
+#pragma unroll 1
+    for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t t = floor | (1u << bit);
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) n += __syncthreads_count(in[k] && c[k] >= t);
+        if (n >= n_slots) floor = t;
+    }
+    if (threadIdx.x == 0) used = 0;
+    __syncthreads();
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (!in[k] || (pass == 0 ? c[k] <= floor : c[k] > floor)) continue;
+            const int i = (int)threadIdx.x + 1024 * k;
+            const int slot = pass == 0 || c[k] == floor ? atomicAdd(&used, 1) : n_slots;
+            table[i] = slot < n_slots ? (int16_t)slot : (int16_t)-1;
+            if (slot < n_slots) slot_cell[slot] = (int16_t)i;
+        }
+        __syncthreads();
+    }
+}
+
 // Dynamic shared memory: n_slots << 2cs counters, then the cell -> slot table (cdim^2 int16).
 template <bool kVec>
 __global__ void __launch_bounds__(kUvThreads, 1)
@@ -609,6 +668,7 @@ __global__ void __launch_bounds__(kUvThreads, 1)
                        int n_slots, uint32_t *__restrict__ ghist)
 {
     extern __shared__ uint32_t sh_hot[];
+    r.load();
     const int n_hot = n_slots << (2 * cs);
     int16_t *stab = reinterpret_cast<int16_t *>(sh_hot + n_hot);
     for (int i = threadIdx.x; i < n_hot; i += blockDim.x) sh_hot[i] = 0u;

@@ -27,35 +27,39 @@ unsigned field_blocks(const potts_context *ctx, int64_t n_lines, int per_sm)
 
 bool field_empty(const Geometry &g) { return g.n_lines == 0 || g.ns == 0; }
 
-// 16-byte loads along a line: lines of a multiple of 4 values and stride, aligned field.
-bool field_vec(const Geometry &g, const float *d_f)
-{
-    return ((uintptr_t)d_f & 15u) == 0 && g.ns % 4 == 0 && g.nstride_w % 4 == 0;
-}
+// 16-byte loads along a line: lines of a stride of a multiple of 4 values, aligned field (the last
+// quad of a line may reach into its padding).
+bool field_vec(const Geometry &g, const float *d_f) { return ((uintptr_t)d_f & 15u) == 0 && g.nstride_w % 4 == 0; }
 
-// min_max (min_max/min_max.cpp:56-81) and, with positive, the min/max of the strictly positive
-// values (uv-hist-kernel.cpp:70-92).  FLT_MAX / -FLT_MAX when there is no such value.
-int minmax_run(potts_context *ctx, const float *d_f, bool positive, float *out_min, float *out_max)
+// Enqueues min_max (min_max/min_max.cpp:56-81) or, with positive, the min/max of the strictly positive
+// values (uv-hist-kernel.cpp:70-92) of a field that is not empty; the two results at *d_res, which stay
+// there until the next range is computed.
+int minmax_enqueue(potts_context *ctx, const float *d_f, bool positive, const float **d_res)
 {
     const Geometry g = field_geometry(ctx);
+    const unsigned nb = field_blocks(ctx, g.n_lines, 8);
+    POTTS_TRY(ensure(ctx, ctx->range, 4 * sizeof(float) + sizeof(float2) * nb));
+    float *res = static_cast<float *>(ctx->range.p);
+    float2 *part = reinterpret_cast<float2 *>(res + 4);
+    auto kern = field_vec(g, d_f) ? (positive ? potts::minmax_partial_kernel<true, true>
+                                              : potts::minmax_partial_kernel<false, true>)
+                                  : (positive ? potts::minmax_partial_kernel<true, false>
+                                              : potts::minmax_partial_kernel<false, false>);
+    kern<<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_f, part);
+    potts::minmax_final_kernel<<<1, potts::kHistThreads, 0, ctx->stream>>>(part, (int)nb, res);
+    ctx->total_launches += 2;
+    POTTS_CUDA(cudaGetLastError());
+    *d_res = res;
+    return POTTS_OK;
+}
+
+// min_max to the host; FLT_MAX / -FLT_MAX when there is no such value.
+int minmax_run(potts_context *ctx, const float *d_f, bool positive, float *out_min, float *out_max)
+{
     float res[2] = {FLT_MAX, -FLT_MAX};
-    if (!field_empty(g)) {
-        const unsigned nb = field_blocks(ctx, g.n_lines, 8);
-        POTTS_TRY(ensure(ctx, ctx->hist, sizeof(float2) * nb + 2 * sizeof(float)));
-        float2 *part = static_cast<float2 *>(ctx->hist.p);
-        float *d_res = reinterpret_cast<float *>(part + nb);
-        const bool vec = ((uintptr_t)d_f & 15u) == 0 && g.ns % 4 == 0 && g.nstride_w % 4 == 0;
-        if (positive && vec)
-            potts::minmax_partial_kernel<true, true><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_f, part);
-        else if (positive)
-            potts::minmax_partial_kernel<true, false><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_f, part);
-        else if (vec)
-            potts::minmax_partial_kernel<false, true><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_f, part);
-        else
-            potts::minmax_partial_kernel<false, false><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_f, part);
-        potts::minmax_final_kernel<<<1, potts::kHistThreads, 0, ctx->stream>>>(part, (int)nb, d_res);
-        ctx->total_launches += 2;
-        POTTS_CUDA(cudaGetLastError());
+    if (!field_empty(field_geometry(ctx))) {
+        const float *d_res;
+        POTTS_TRY(minmax_enqueue(ctx, d_f, positive, &d_res));
         POTTS_CUDA(cudaMemcpyAsync(res, d_res, sizeof(res), cudaMemcpyDeviceToHost, ctx->stream));
         POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
     }
@@ -64,28 +68,23 @@ int minmax_run(potts_context *ctx, const float *d_f, bool positive, float *out_m
     return POTTS_OK;
 }
 
-// The ranges of uv_hist_auto in one pass: out = (min u, max u, min v, max v) over every u and the
-// strictly positive v (uv-hist-kernel.cpp:70-98); FLT_MAX / -FLT_MAX where there is no value.
-int minmax_pair_run(potts_context *ctx, const float *d_u, const float *d_v, float *out)
+// Enqueues the ranges of uv_hist_auto in one pass over fields that are not empty: (min u, max u, min
+// v, max v) over every u and the strictly positive v (uv-hist-kernel.cpp:70-98) at *d_res.
+int minmax_pair_enqueue(potts_context *ctx, const float *d_u, const float *d_v, const float **d_res)
 {
     const Geometry g = field_geometry(ctx);
-    float res[4] = {FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX};
-    if (!field_empty(g)) {
-        const unsigned nb = field_blocks(ctx, g.n_lines, 8);
-        POTTS_TRY(ensure(ctx, ctx->hist, sizeof(float4) * nb + 4 * sizeof(float)));
-        float4 *part = static_cast<float4 *>(ctx->hist.p);
-        float *d_res = reinterpret_cast<float *>(part + nb);
-        if (field_vec(g, d_u) && field_vec(g, d_v))
-            potts::minmax_pair_partial_kernel<true><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_u, d_v, part);
-        else
-            potts::minmax_pair_partial_kernel<false><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_u, d_v, part);
-        potts::minmax_pair_final_kernel<<<1, potts::kHistThreads, 0, ctx->stream>>>(part, (int)nb, d_res);
-        ctx->total_launches += 2;
-        POTTS_CUDA(cudaGetLastError());
-        POTTS_CUDA(cudaMemcpyAsync(res, d_res, sizeof(res), cudaMemcpyDeviceToHost, ctx->stream));
-        POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
-    }
-    std::copy(res, res + 4, out);
+    const unsigned nb = field_blocks(ctx, g.n_lines, 8);
+    POTTS_TRY(ensure(ctx, ctx->range, sizeof(float4) * ((size_t)nb + 1)));
+    float *res = static_cast<float *>(ctx->range.p);
+    float4 *part = static_cast<float4 *>(ctx->range.p) + 1;
+    if (field_vec(g, d_u) && field_vec(g, d_v))
+        potts::minmax_pair_partial_kernel<true><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_u, d_v, part);
+    else
+        potts::minmax_pair_partial_kernel<false><<<nb, potts::kHistThreads, 0, ctx->stream>>>(g, d_u, d_v, part);
+    potts::minmax_pair_final_kernel<<<1, potts::kHistThreads, 0, ctx->stream>>>(part, (int)nb, res);
+    ctx->total_launches += 2;
+    POTTS_CUDA(cudaGetLastError());
+    *d_res = res;
     return POTTS_OK;
 }
 
@@ -94,11 +93,11 @@ int minmax_pair_run(potts_context *ctx, const float *d_u, const float *d_v, floa
 int grad_magn_tiled(potts_context *ctx, const Geometry &g, const float *d_u, float *d_v)
 {
     using T = potts::GmTile;
-    // segments of 64 columns; of 16 when 64 leave fewer than four blocks per multiprocessor (decided
-    // once per mapping and slice count)
+    // the column segment is chosen once per mapping and slice count
     if (ctx->gm_segment == 0 || ctx->gm_ns != g.ns) {
-        const size_t items = work_items(ctx->mapping.m, g.ns, TileChoice{T::TR, T::TN, 1, 64}).size();
-        ctx->gm_segment = items < (size_t)4 * std::max(ctx->n_sm, 1) ? 16 : 64;
+        const potts_mapping &m = ctx->mapping.m;
+        march_time({{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, T::TR, T::TN,
+                   potts::kGmBlocks * std::max(ctx->n_sm, 1), 0, &ctx->gm_segment);
         ctx->gm_ns = g.ns;
     }
     POTTS_TRY(plan_tiles(ctx, g.ns, TileChoice{T::TR, T::TN, 1, ctx->gm_segment}));
@@ -124,12 +123,13 @@ int grad_magn_tiled(potts_context *ctx, const Geometry &g, const float *d_u, flo
 // grad_magn (grad-magn/grad_magn.cpp:60-79): v at every in-mask voxel.  Fields of 16-byte lines
 // and stride march along the columns (grad_magn_tiled: 0.76 ms at 768^2 x 1024 against 1.09 ms
 // for one warp per line with 16-byte loads of the line and its four neighbour lines, which
-// waited on those loads); others take one thread per voxel.
+// waited on those loads); others take one thread per voxel (four slices per thread with 16-byte loads of
+// the line and its neighbours measured 75 against 78 us at 317 x 300 x 300: both wait for L2).
 int grad_magn_run(potts_context *ctx, const float *d_u, float *d_v)
 {
     const Geometry g = field_geometry(ctx);
     if (field_empty(g)) return POTTS_OK;
-    if (field_vec(g, d_u) && field_vec(g, d_v)) return grad_magn_tiled(ctx, g, d_u, d_v);
+    if (g.ns % 4 == 0 && field_vec(g, d_u) && field_vec(g, d_v)) return grad_magn_tiled(ctx, g, d_u, d_v);
     potts::grad_magn_kernel<<<field_blocks(ctx, g.n_lines, 8), potts::kHistThreads, 0, ctx->stream>>>(g, d_u, d_v);
     ctx->total_launches += 1;
     POTTS_CUDA(cudaGetLastError());
@@ -139,9 +139,11 @@ int grad_magn_run(potts_context *ctx, const float *d_u, float *d_v)
 constexpr int kHist1dSharedMax = 50 * 1024;  // bins kept in shared memory (200 KB)
 constexpr int kHist1dPerWarpMax = 100 * 1024;  // shared bytes of per-warp copies (two blocks per SM)
 
-// calc_hist (calc_hist/calc_hist.cpp:93-138): counts of nb bins over [rs, re] to the host.
-int hist1d_run(potts_context *ctx, const float *d_f, float rs, float re, int nb, float delta, uint64_t seed,
-               uint32_t *h_counts)
+// calc_hist (calc_hist/calc_hist.cpp:93-138): counts of nb bins over [rs, re] to the host; with
+// d_range the two ends are read from device memory, where an enqueued pass leaves them, and copied
+// to h_range.
+int hist1d_run(potts_context *ctx, const float *d_f, float rs, float re, const float *d_range, int nb, float delta,
+               uint64_t seed, uint32_t *h_counts, float *h_range)
 {
     const Geometry g = field_geometry(ctx);
     POTTS_TRY(ensure(ctx, ctx->hist, sizeof(uint32_t) * nb));
@@ -160,8 +162,8 @@ int hist1d_run(potts_context *ctx, const float *d_f, float rs, float re, int nb,
             const bool vec = field_vec(g, d_f);
             auto launch = [&](auto kern) -> int {
                 POTTS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-                kern<<<blocks, potts::kHistThreads, smem, ctx->stream>>>(g, d_f, rs, re, nb, copies, delta, seed,
-                                                                         d_counts);
+                kern<<<blocks, potts::kHistThreads, smem, ctx->stream>>>(g, d_f, rs, re, d_range, nb, copies, delta,
+                                                                         seed, d_counts);
                 return POTTS_OK;
             };
             if (jitter)
@@ -172,17 +174,28 @@ int hist1d_run(potts_context *ctx, const float *d_f, float rs, float re, int nb,
             const unsigned blocks = field_blocks(ctx, g.n_lines, 8);
             if (jitter)
                 potts::hist1d_global_kernel<true><<<blocks, potts::kHistThreads, 0, ctx->stream>>>(
-                    g, d_f, rs, re, nb, delta, seed, d_counts);
+                    g, d_f, rs, re, d_range, nb, delta, seed, d_counts);
             else
                 potts::hist1d_global_kernel<false><<<blocks, potts::kHistThreads, 0, ctx->stream>>>(
-                    g, d_f, rs, re, nb, delta, seed, d_counts);
+                    g, d_f, rs, re, d_range, nb, delta, seed, d_counts);
         }
         ctx->total_launches += 1;
         POTTS_CUDA(cudaGetLastError());
     }
+    if (d_range) POTTS_CUDA(cudaMemcpyAsync(h_range, d_range, 2 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     POTTS_CUDA(cudaMemcpyAsync(h_counts, d_counts, sizeof(uint32_t) * nb, cudaMemcpyDeviceToHost, ctx->stream));
     POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
     return POTTS_OK;
+}
+
+// calc_hist.cpp:129-135: counts / (in-mask voxels x bin width), in double; density may be null.
+void hist_density(const potts_context *ctx, float rs, float re, uint32_t nb, const uint32_t *counts, double *density)
+{
+    if (!density) return;
+    const double bin_width = ((double)re - (double)rs) / nb;
+    const double voxels = (double)ctx->mapping.n_lines * (double)ctx->mapping.m.n_images;
+    const double scale = 1.0 / (voxels * bin_width);
+    for (uint32_t i = 0; i < nb; ++i) density[i] = counts[i] * scale;
 }
 
 // Row stride and span of the 2-D histogram (uv-hist-kernel.cpp:112-118): rows padded to 128 bytes.
@@ -190,7 +203,7 @@ uint32_t uv_stride(int nb) { return (uint32_t)((nb + 31) / 32 * 32); }
 uint64_t uv_span(int nb) { return (uint64_t)(nb - 1) * uv_stride(nb) + (uint64_t)nb; }
 
 // The 2-D histogram through the hot-cell kernels (kernels_hist.cuh): a coarse pass over every
-// 8th line, the densest cells to shared memory, the rest to global atomics.
+// step-th line, the densest cells to shared memory, the rest to global atomics.
 int uv_hist_hot(potts_context *ctx, const Geometry &g, const float *d_u, const float *d_v, const potts::UvRange &r,
                 uint32_t *d_hist)
 {
@@ -219,21 +232,9 @@ int uv_hist_hot(potts_context *ctx, const Geometry &g, const float *d_u, const f
                                                                                         step, d_coarse);
     ctx->total_launches += 1;
     POTTS_CUDA(cudaGetLastError());
-    std::vector<uint32_t> counts((size_t)cells);
-    POTTS_CUDA(cudaMemcpyAsync(counts.data(), d_coarse, sizeof(uint32_t) * cells, cudaMemcpyDeviceToHost,
-                               ctx->stream));
-    POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
-    std::vector<int> order((size_t)cells);
-    for (int i = 0; i < cells; ++i) order[(size_t)i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return counts[(size_t)a] > counts[(size_t)b]; });
-    std::vector<int16_t> table((size_t)cells, (int16_t)-1), slot_cell((size_t)std::max(n_slots, 1), (int16_t)0);
-    for (int s = 0; s < n_slots; ++s) {
-        table[(size_t)order[(size_t)s]] = (int16_t)s;
-        slot_cell[(size_t)s] = (int16_t)order[(size_t)s];
-    }
-    POTTS_CUDA(cudaMemcpyAsync(d_table, table.data(), sizeof(int16_t) * cells, cudaMemcpyHostToDevice, ctx->stream));
-    POTTS_CUDA(cudaMemcpyAsync(d_cells, slot_cell.data(), sizeof(int16_t) * n_slots, cudaMemcpyHostToDevice,
-                               ctx->stream));
+    potts::uv_select_kernel<<<1, 1024, 0, ctx->stream>>>(d_coarse, cells, n_slots, d_table, d_cells);
+    ctx->total_launches += 1;
+    POTTS_CUDA(cudaGetLastError());
     const int smem = (int)(sizeof(uint32_t) * ((size_t)n_slots << (2 * cs)) + sizeof(int16_t) * cells);
     auto hot = vec ? potts::uv_hist_hot_kernel<true> : potts::uv_hist_hot_kernel<false>;
     POTTS_CUDA(cudaFuncSetAttribute(hot, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -243,13 +244,13 @@ int uv_hist_hot(potts_context *ctx, const Geometry &g, const float *d_u, const f
                                                            d_hist);
     ctx->total_launches += 1;
     POTTS_CUDA(cudaGetLastError());
-    // the host vectors above are pageable: wait for the copies before they go out of scope
-    POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
     return POTTS_OK;
 }
 
-// uv_hist (uv-hist-kernel.cpp:100-197): the 2-D histogram of (u, v) to the host.
-int uv_hist_run(potts_context *ctx, const float *d_u, const float *d_v, const potts::UvRange &r, uint32_t *h_hist)
+// uv_hist (uv-hist-kernel.cpp:100-197): the 2-D histogram of (u, v) to the host; ranges in device
+// memory (r.dev) are copied to h_range.
+int uv_hist_run(potts_context *ctx, const float *d_u, const float *d_v, const potts::UvRange &r, uint32_t *h_hist,
+                float *h_range)
 {
     const Geometry g = field_geometry(ctx);
     const uint64_t span = uv_span(r.nb);
@@ -257,6 +258,7 @@ int uv_hist_run(potts_context *ctx, const float *d_u, const float *d_v, const po
     uint32_t *d_hist = static_cast<uint32_t *>(ctx->hist.p);
     POTTS_CUDA(cudaMemsetAsync(d_hist, 0, sizeof(uint32_t) * span, ctx->stream));
     if (!field_empty(g)) POTTS_TRY(uv_hist_hot(ctx, g, d_u, d_v, r, d_hist));
+    if (r.dev) POTTS_CUDA(cudaMemcpyAsync(h_range, r.dev, 4 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     POTTS_CUDA(cudaMemcpyAsync(h_hist, d_hist, sizeof(uint32_t) * span, cudaMemcpyDeviceToHost, ctx->stream));
     POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
     return POTTS_OK;

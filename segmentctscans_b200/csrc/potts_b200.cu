@@ -211,7 +211,8 @@ struct potts_context {
     MappingCopy mapping;  // last mapping whose line table is on the device
     bool mapping_valid = false;
     DevBuf lines, state, dq, energy, partial, host_u, host_res, host_labels, ustage, err;
-    DevBuf hist;      // min/max partials and histogram counters of the label-finding inputs
+    DevBuf hist;      // histogram counters of the label-finding inputs
+    DevBuf range;     // min/max results and partials of the label-finding inputs
     DevBuf hist_aux;  // coarse cell counts and cell tables of the 2-D histogram
     DevBuf io, io_tables;  // archive payload / raw label box staging, mask tables of the box kernel
     float *pinned_dq = nullptr;
@@ -1353,7 +1354,7 @@ void potts_context_destroy(potts_context *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (DevBuf *b : {&ctx->lines, &ctx->state, &ctx->dq, &ctx->energy, &ctx->partial, &ctx->host_u,
                       &ctx->host_res, &ctx->host_labels, &ctx->ustage, &ctx->err, &ctx->cols, &ctx->work, &ctx->vols,
-                      &ctx->hist, &ctx->hist_aux, &ctx->io, &ctx->io_tables, &ctx->pctl})
+                      &ctx->hist, &ctx->hist_aux, &ctx->range, &ctx->io, &ctx->io_tables, &ctx->pctl})
         if (b->p) cudaFree(b->p);
     if (ctx->pinned_dq) cudaFreeHost(ctx->pinned_dq);
     for (cudaEvent_t e : ctx->seg_ev) cudaEventDestroy(e);
@@ -1808,14 +1809,8 @@ int potts_calc_hist(potts_context *ctx, const potts_mapping *map, const float *d
     if (!std::isfinite(jitter) || jitter < 0.0f) return fail(POTTS_EINVAL, "jitter must be finite and >= 0");
     POTTS_CUDA(cudaSetDevice(ctx->device));
     POTTS_TRY(upload_lines(ctx, map));
-    POTTS_TRY(hist1d_run(ctx, d_field, range_start, range_end, (int)nbins, jitter, seed, out_counts));
-    if (out_density) {
-        // calc_hist.cpp:129-135: counts / (in-mask voxels x bin width), in double
-        const double bin_width = ((double)range_end - (double)range_start) / nbins;
-        const double voxels = (double)ctx->mapping.n_lines * (double)ctx->mapping.m.n_images;
-        const double scale = 1.0 / (voxels * bin_width);
-        for (uint32_t i = 0; i < nbins; ++i) out_density[i] = out_counts[i] * scale;
-    }
+    POTTS_TRY(hist1d_run(ctx, d_field, range_start, range_end, nullptr, (int)nbins, jitter, seed, out_counts, nullptr));
+    hist_density(ctx, range_start, range_end, nbins, out_counts, out_density);
     return POTTS_OK;
 }
 
@@ -1825,8 +1820,20 @@ int potts_calc_hist_auto(potts_context *ctx, const potts_mapping *map, const flo
 {
     if (!ctx || !map || !d_field || !out_counts || !out_min || !out_max) return fail(POTTS_EINVAL, "NULL argument");
     POTTS_TRY(check_nbins(nbins));
-    POTTS_TRY(potts_min_max(ctx, map, d_field, out_min, out_max));
-    return potts_calc_hist(ctx, map, d_field, *out_min, *out_max, nbins, jitter, seed, out_counts, out_density);
+    POTTS_CUDA(cudaSetDevice(ctx->device));
+    POTTS_TRY(upload_lines(ctx, map));
+    if (field_empty(field_geometry(ctx)) || !std::isfinite(jitter) || jitter < 0.0f) {
+        POTTS_TRY(minmax_run(ctx, d_field, false, out_min, out_max));
+        return potts_calc_hist(ctx, map, d_field, *out_min, *out_max, nbins, jitter, seed, out_counts, out_density);
+    }
+    // the histogram reads the range where the first pass leaves it: one wait for both
+    const float *d_range;
+    float range[2];
+    POTTS_TRY(minmax_enqueue(ctx, d_field, false, &d_range));
+    POTTS_TRY(hist1d_run(ctx, d_field, 0.0f, 0.0f, d_range, (int)nbins, jitter, seed, out_counts, range));
+    *out_min = range[0], *out_max = range[1];
+    hist_density(ctx, range[0], range[1], nbins, out_counts, out_density);
+    return POTTS_OK;
 }
 
 uint32_t potts_uv_hist_stride(uint32_t nbins) { return nbins ? uv_stride((int)nbins) : 0u; }
@@ -1840,8 +1847,8 @@ int potts_uv_hist(potts_context *ctx, const potts_mapping *map, const float *d_u
     POTTS_TRY(check_nbins(nbins));
     POTTS_CUDA(cudaSetDevice(ctx->device));
     POTTS_TRY(upload_lines(ctx, map));
-    const potts::UvRange r{u_start, u_end, v_start, v_end, (int)nbins, (int)uv_stride((int)nbins)};
-    return uv_hist_run(ctx, d_u, d_v, r, out_hist);
+    const potts::UvRange r{u_start, u_end, v_start, v_end, (int)nbins, (int)uv_stride((int)nbins), nullptr};
+    return uv_hist_run(ctx, d_u, d_v, r, out_hist, nullptr);
 }
 
 int potts_uv_hist_auto(potts_context *ctx, const potts_mapping *map, const float *d_u, const float *d_v,
@@ -1852,9 +1859,11 @@ int potts_uv_hist_auto(potts_context *ctx, const potts_mapping *map, const float
     // uv-hist-kernel.cpp:70-98: v over its strictly positive values, u over all (one pass)
     POTTS_CUDA(cudaSetDevice(ctx->device));
     POTTS_TRY(upload_lines(ctx, map));
-    POTTS_TRY(minmax_pair_run(ctx, d_u, d_v, out_ranges));
-    return potts_uv_hist(ctx, map, d_u, d_v, out_ranges[0], out_ranges[1], out_ranges[2], out_ranges[3], nbins,
-                         out_hist);
+    potts::UvRange r{FLT_MAX, -FLT_MAX, FLT_MAX, -FLT_MAX, (int)nbins, (int)uv_stride((int)nbins), nullptr};
+    const float none[4] = {r.us, r.ue, r.vs, r.ve};
+    std::copy(none, none + 4, out_ranges);
+    if (!field_empty(field_geometry(ctx))) POTTS_TRY(minmax_pair_enqueue(ctx, d_u, d_v, &r.dev));
+    return uv_hist_run(ctx, d_u, d_v, r, out_hist, out_ranges);
 }
 
 int potts_archive_read_header(const uint8_t *bytes, uint64_t n_bytes, int elem, potts_archive_info *info,
