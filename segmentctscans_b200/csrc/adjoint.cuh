@@ -10,6 +10,7 @@
 
 struct potts_tape {
     potts_context *ctx = nullptr;
+    std::shared_ptr<TapePool> pool;  // of the context, which this tape may outlive
     MappingCopy mc;
     Geometry g{};
     DevBuf lines, ckpt, seg, A, X, Q, P, grads, loss;
@@ -23,15 +24,31 @@ struct potts_tape {
 
 namespace {
 
+void tape_bufs(potts_tape *t, DevBuf *(&bufs)[kTapeBufs])
+{
+    DevBuf *const all[kTapeBufs] = {&t->lines, &t->ckpt, &t->seg, &t->A, &t->X, &t->Q, &t->P, &t->grads, &t->loss};
+    std::copy(all, all + kTapeBufs, bufs);
+}
+
 void tape_free(potts_tape *t)
 {
     if (!t) return;
-    if (t->ctx) {
+    if (t->pool && t->pool->open) {
         cudaSetDevice(t->ctx->device);
         cudaStreamSynchronize(t->ctx->stream);
     }
-    for (DevBuf *d : {&t->lines, &t->ckpt, &t->seg, &t->A, &t->X, &t->Q, &t->P, &t->grads, &t->loss})
-        if (d->p) cudaFree(d->p);
+    DevBuf *bufs[kTapeBufs];
+    tape_bufs(t, bufs);
+    size_t bytes = 0;
+    for (DevBuf *d : bufs) bytes += d->bytes;
+    // kept in place of an earlier tape's (the stream is idle: nothing uses them)
+    if (t->pool && t->pool->open && bytes <= kTapePoolBytes) {
+        t->pool->give_back();
+        for (int i = 0; i < kTapeBufs; ++i) t->pool->buf[i] = *bufs[i];
+    } else {
+        for (DevBuf *d : bufs)
+            if (d->p) cudaFree(d->p);
+    }
     delete t;
 }
 
@@ -171,9 +188,25 @@ int tape_alloc(potts_tape *t)
     potts_context *ctx = t->ctx;
     const size_t state = sizeof(float) * tape_state_floats(t);
     const size_t pw = sizeof(float) * (size_t)t->g.plane_w;
+    // an earlier tape's buffers where each is large enough, and at most twice what is needed; else its
+    // memory is given back first
+    const size_t sizes[kTapeBufs] = {0, state * (size_t)t->n_ckpt, state * ((size_t)t->every + 1),
+                                     pw * (size_t)(t->K - 1), pw * 3 * (size_t)(t->K - 1), pw * (size_t)t->K,
+                                     pw * 3 * (size_t)t->K, 0, 0};
+    DevBuf *bufs[kTapeBufs];
+    tape_bufs(t, bufs);
+    bool fits = t->pool->bytes() > 0;
+    for (int i = 1; i < 7; ++i) {
+        const size_t have = t->pool->buf[i].bytes;
+        fits = fits && have >= sizes[i] && have / 2 <= sizes[i];
+    }
+    if (fits) {
+        for (int i = 1; i < kTapeBufs; ++i) std::swap(*bufs[i], t->pool->buf[i]);
+    }
+    t->pool->give_back();
     size_t free_b = 0, total_b = 0;
     POTTS_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const size_t need = state * ((size_t)t->n_ckpt + (size_t)t->every + 1) +
+    const size_t need = fits ? 0 : state * ((size_t)t->n_ckpt + (size_t)t->every + 1) +
                         pw * ((size_t)(t->K - 1) * 4 + (size_t)t->K * 4) + (size_t(256) << 20);
     if (need > free_b) return fail(POTTS_ENOMEM, "the checkpoints and the segment's states do not fit in memory");
     POTTS_TRY(ensure(ctx, t->ckpt, state * (size_t)t->n_ckpt));

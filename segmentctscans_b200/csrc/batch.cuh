@@ -296,6 +296,7 @@ int batch_build(potts_batch *b)
         b->voxels += bv.voxels;
     }
     size_t free_b = 0, total_b = 0;
+    ctx->tape_pool->give_back();
     POTTS_CUDA(cudaMemGetInfo(&free_b, &total_b));
     if (state + (size_t(512) << 20) > free_b) return fail(POTTS_ENOMEM, "the batch's state does not fit in memory");
     b->state_bytes = state;

@@ -200,6 +200,32 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// Device buffers of a finished tape, kept by its context for the next one: allocating and freeing
+// several GB costs more than a tenth of a forward and backward pass (192^3, 40 iterations: 9 of 47 ms).
+// Bounded: the buffers of one tape, at most kTapePoolBytes.  Given back when the context is destroyed
+// and before the library plans a solve, a batch, a shard or a tape by the free memory, or when an
+// allocation fails.  A tape may outlive its context: it shares the pool, which is then closed.
+constexpr int kTapeBufs = 9;
+constexpr size_t kTapePoolBytes = size_t(8) << 30;
+struct TapePool {
+    DevBuf buf[kTapeBufs];
+    bool open = true;
+
+    size_t bytes() const
+    {
+        size_t n = 0;
+        for (const DevBuf &b : buf) n += b.bytes;
+        return n;
+    }
+    void give_back()
+    {
+        for (DevBuf &b : buf) {
+            if (b.p) cudaFree(b.p);  // waits for work on the device that may still use it
+            b = DevBuf{};
+        }
+    }
+};
+
 }  // namespace
 
 struct potts_context {
@@ -238,6 +264,7 @@ struct potts_context {
     int loop_iters = 0;  // iterations inside the event pairs
     // control words of persistent fused launches (item counters per iteration, grid barrier)
     DevBuf pctl;
+    std::shared_ptr<TapePool> tape_pool = std::make_shared<TapePool>();
 };
 
 struct potts_field {
@@ -293,7 +320,12 @@ int ensure(potts_context *ctx, DevBuf &b, size_t bytes)
         b.bytes = 0;
     }
     if (bytes == 0) return POTTS_OK;
-    POTTS_CUDA(cudaMalloc(&b.p, bytes));
+    if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        b.p = nullptr;
+        ctx->tape_pool->give_back();
+        POTTS_CUDA(cudaMalloc(&b.p, bytes));
+    }
     b.bytes = bytes;
     return POTTS_OK;
 }
@@ -312,7 +344,7 @@ int release(potts_context *ctx, DevBuf &b)
 size_t cached_bytes(const potts_context *ctx)
 {
     return ctx->state.bytes + ctx->partial.bytes + ctx->host_u.bytes + ctx->host_res.bytes + ctx->host_labels.bytes +
-           ctx->ustage.bytes + ctx->hist.bytes + ctx->io.bytes + ctx->io_tables.bytes;
+           ctx->ustage.bytes + ctx->hist.bytes + ctx->io.bytes + ctx->io_tables.bytes + ctx->tape_pool->bytes();
 }
 
 int upload_lines(potts_context *ctx, const potts_mapping *map)
@@ -959,6 +991,7 @@ int solve_k(potts_context *ctx, const float *d_u, const float *ci, float lam, fl
     // staging buffers are scratch of earlier calls: the solve gets their memory.
     POTTS_TRY(release(ctx, ctx->io));
     POTTS_TRY(release(ctx, ctx->io_tables));
+    ctx->tape_pool->give_back();
     size_t free_b = 0, total_b = 0;
     POTTS_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t margin = size_t(512) << 20;
@@ -1356,6 +1389,8 @@ void potts_context_destroy(potts_context *ctx)
                       &ctx->host_res, &ctx->host_labels, &ctx->ustage, &ctx->err, &ctx->cols, &ctx->work, &ctx->vols,
                       &ctx->hist, &ctx->hist_aux, &ctx->range, &ctx->io, &ctx->io_tables, &ctx->pctl})
         if (b->p) cudaFree(b->p);
+    ctx->tape_pool->give_back();
+    ctx->tape_pool->open = false;
     if (ctx->pinned_dq) cudaFreeHost(ctx->pinned_dq);
     for (cudaEvent_t e : ctx->seg_ev) cudaEventDestroy(e);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -1396,6 +1431,11 @@ int potts_field_create(potts_context *ctx, const potts_mapping *map, potts_field
     cudaSetDevice(ctx->device);
     const size_t bytes = sizeof(float) * (size_t)std::max<uint64_t>(f->mapping.span, 1);
     cudaError_t e = cudaMalloc(&f->d, bytes);
+    if (e != cudaSuccess && ctx->tape_pool->bytes() > 0) {
+        cudaGetLastError();
+        ctx->tape_pool->give_back();
+        e = cudaMalloc(&f->d, bytes);
+    }
     if (e != cudaSuccess) {
         delete f;
         return fail(e == cudaErrorMemoryAllocation ? POTTS_ENOMEM : POTTS_ECUDA, cudaGetErrorString(e));
@@ -1686,6 +1726,7 @@ int potts_forward_ckpt(potts_context *ctx, const potts_mapping *map, const float
     POTTS_CUDA(cudaSetDevice(ctx->device));
     auto *t = new potts_tape();
     t->ctx = ctx;
+    t->pool = ctx->tape_pool;
     int rc = copy_mapping(map, t->mc);
     if (rc == POTTS_OK) {
         t->K = K;
