@@ -125,6 +125,9 @@ struct TileShape {
     static constexpr int OFF_BAR = OFF_COLS + al((MAX_SEGMENT + 3) * 16);
     static constexpr int SMEM = OFF_BAR + 3 * D * 8 + 16;  // + abort flag
     static constexpr int SMEM_ALLOC = SMEM + 128;  // room to align the base to 128 bytes
+    // blocks per multiprocessor: two of at most 256 threads (128 registers each) where both fit its
+    // 228 KB (1 KB of each block is reserved)
+    static constexpr int BLOCKS = THREADS <= 256 && 2 * (SMEM_ALLOC + 1024) <= 228 * 1024 ? 2 : 1;
     static_assert((VPT == 2 || VPT == 4) && NT % VPT == 0 && R + 1 <= 32, "tile shape");
     static_assert(MAIN % 32 == 0, "row threads fill whole warps");
     static_assert(SMEM_ALLOC <= 227 * 1024, "shared memory of one block");
@@ -969,7 +972,7 @@ __device__ __forceinline__ TiledSmem<K, R, NT, VPT, ST> tiled_smem()
 // turns (Xi^m, V^{m-1}) in half `in` into (Xi^{m+1}, V^m) in half in ^ 1;
 // it = m - 1.
 template <int K, int R, int NT, int VPT, typename ST, bool FAST>
-__global__ void __launch_bounds__(TileShape<K, R, NT, VPT, ST>::THREADS, 1)
+__global__ void __launch_bounds__(TileShape<K, R, NT, VPT, ST>::THREADS, TileShape<K, R, NT, VPT, ST>::BLOCKS)
     fused_tiled_kernel(const FusedVolume<K, ST> *__restrict__ vols, const int4 *__restrict__ work,
                        const int *__restrict__ work_vol, int in, int it, float tau2, DykstraThresholds thr, int *err)
 {
@@ -1019,7 +1022,7 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t target)
 // into the other half, like fused_tiled_kernel.  The result does not depend on
 // the grid size or the order in which blocks take items.
 template <int K, int R, int NT, int VPT, typename ST, bool FAST>
-__global__ void __launch_bounds__(TileShape<K, R, NT, VPT, ST>::THREADS, 1)
+__global__ void __launch_bounds__(TileShape<K, R, NT, VPT, ST>::THREADS, TileShape<K, R, NT, VPT, ST>::BLOCKS)
     fused_persistent_kernel(const FusedVolume<K, ST> *__restrict__ vols, const int4 *__restrict__ work,
                             const int *__restrict__ work_vol, int n_work, int in0, int it0, int n_iters, float tau2,
                             DykstraThresholds thr, int *err, uint32_t *ctl)

@@ -6,6 +6,7 @@
 #include <nccl.h>
 
 #include <algorithm>
+#include <array>
 #include <memory>
 #include <mutex>
 #include <cfloat>
@@ -582,6 +583,14 @@ double march_time(const std::vector<MarchVolume> &vols, int rows, int slices, in
     return best_time;
 }
 
+// Blocks per multiprocessor of each compiled shape.
+template <int K, typename ST, size_t... I>
+std::array<int, sizeof...(I)> shape_blocks(std::index_sequence<I...>)
+{
+    using TS = ShapesOf<K, ST>;
+    return {potts::TileShape<K, TS::r[I], TS::t[I], TS::v[I], ST>::BLOCKS...};
+}
+
 // Tile shape and segment length: the options', or those with the least expected
 // time over the volumes (a shape's time per voxel times its march_time: ragged
 // slices and rows cost as much as full ones).  The results depend on neither.
@@ -591,6 +600,7 @@ int choose_tile(const potts_options &o, const std::vector<MarchVolume> &vols, in
     using TS = ShapesOf<K, ST>;
     if (o.segment_cols > 64) return fail(POTTS_EINVAL, "segment_cols must be <= 64");
     const bool named = o.tile_rows > 0 || o.tile_slices > 0 || o.tile_vpt > 0;
+    const auto blocks = shape_blocks<K, ST>(std::make_index_sequence<(size_t)TS::n>());
     double best = -1.0;
     for (int i = 0; i < (named ? TS::named : TS::n); ++i) {
         if (named && !((o.tile_rows <= 0 || o.tile_rows == TS::r[i]) && (o.tile_slices <= 0 || o.tile_slices == TS::t[i]) &&
@@ -598,8 +608,10 @@ int choose_tile(const potts_options &o, const std::vector<MarchVolume> &vols, in
             continue;
         int segment = 64;
         const int weight = o.arith == POTTS_ARITH_FAST ? TS::fast[i] : TS::exact[i];
-        const double time = march_time(vols, TS::r[i], TS::t[i], std::max(n_sm, 1), o.segment_cols, &segment) *
-                            (weight * TS::r[i] * TS::t[i]);
+        // b blocks on a multiprocessor share its rate
+        const int b = blocks[(size_t)i];
+        const double time = march_time(vols, TS::r[i], TS::t[i], b * std::max(n_sm, 1), o.segment_cols, &segment) *
+                            (weight * TS::r[i] * TS::t[i] * b);
         if (best < 0.0 || time < best) {
             best = time;
             *tc = TileChoice{TS::r[i], TS::t[i], TS::v[i], segment};
