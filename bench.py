@@ -942,14 +942,14 @@ def run_tv(args, dist_: Dist) -> None:
     value = dist_.reduce(float(vox) * iters * args.steps, "sum") / t_max / 1e9
     launch_s = sum(s.loop_ms for s in stats) / 1000.0 / max(sum(s.loop_launches for s in stats), 1)
     iter_s = sum(s.loop_ms for s in stats) / 1000.0 / max(sum(s.loop_iters for s in stats), 1)
-    # tiled: xi (3) and the differences of g (3) in, xi (3) out; per-voxel fused: xi (3) and g in,
+    # tiled and per-voxel fused: xi (3) and g in, xi (3) out;
     # xi (3) out; split: div reads xi (3), writes v; grad reads v, g, xi (3), writes xi (3)
-    bpv = {0: 36, 1: 48, 2: 28}[variant]
+    bpv = {0: 28, 1: 48, 2: 28}[variant]
     achieved = bpv * vox / iter_s / 1e9
     peaks = measured_peaks()
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": None,
-                "kernel": {0: "potts::tv_tiled_kernel<8,128>", 1: "potts::tv_div_kernel + tv_grad_kernel (average launch)",
+                "kernel": {0: "potts::tv_tiled_kernel", 1: "potts::tv_div_kernel + tv_grad_kernel (average launch)",
                            2: "potts::tv_fused_kernel"}[variant],
                 "bytes_per_voxel_iter": bpv,
                 "avg_launch_ms": round(launch_s * 1000, 4),
@@ -1216,7 +1216,7 @@ def run_labels(args, dist_: Dist) -> None:
                    "frac": round(algo[k] / (avg[k] / 1000.0) / 1e9 / peaks["hbm_gbs"], 4),
                    "bytes_per_call": algo[k]} for k in avg}
     # the dominant call: uv_hist_auto (its ranges in one pass over u and v, the coarse cell count
-    # over every 8th line, the hot-cell histogram), against its 16 B per voxel
+    # over a sample of the lines, the hot-cell histogram), against its 16 B per voxel
     roofline = {"bound": "hbm", "achieved": kernels["uv_hist_auto"]["gbs"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": kernels["uv_hist_auto"]["frac"], "traffic": None,
                 "kernel": "uv_hist_auto: potts::minmax_pair_partial_kernel, potts::uv_coarse_kernel, "

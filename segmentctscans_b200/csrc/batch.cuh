@@ -306,7 +306,7 @@ int batch_build(potts_batch *b)
     if (stage > 0) POTTS_TRY(ensure(ctx, b->ustage, sizeof(float) * stage));
     if (b->opts.track_dq && b->iters > 0)
         POTTS_TRY(ensure(ctx, b->dq, sizeof(float) * (size_t)b->iters * b->vols.size()));
-    POTTS_TRY(ensure(ctx, ctx->err, sizeof(int)));
+    POTTS_TRY(ensure(ctx, ctx->err, kErrBytes));
     for (BatchVolume &bv : b->vols) {
         int4 *dl = static_cast<int4 *>(b->lines.p) + bv.lines_off;
         if (bv.mc.n_lines > 0)

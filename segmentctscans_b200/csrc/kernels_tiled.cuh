@@ -453,7 +453,7 @@ __device__ __forceinline__ float get_slot(const float &v, int) { return v; }
 // of them are free.  A sweep is a serial chain of about a hundred dependent
 // operations, so its latency and the instructions around it (polling, taking,
 // storing), not the arithmetic, set the warp's rate: the two voxels share both,
-// two sweeps share the polling (at K = 4 that loop spilled), and the warp sleeps
+// two sweeps share the polling (where that does not spill), and the warp sleeps
 // while fewer than half of its slots hold a voxel and more are to come.  At 512 x
 // 512 x 256, K = 3, 13 % of the voxels in the loop and 4.5 sweeps each (iterations
 // 2 to 40): 1.016 -> 0.799 ms per iteration in the fast arithmetic (one voxel per
@@ -472,7 +472,9 @@ __device__ __forceinline__ void dykstra_worker(const TiledSmem<K, R, NT, VPT, ST
     constexpr int kPairs = K * (K - 1) / 2;
     constexpr int kSlots = K <= 4 ? 2 : 1;
     constexpr int kAll = 32 * kSlots, kRefill = kAll / 4, kFreeMax = kAll / 2;
-    constexpr int kSweeps = K <= 3 ? 2 : 1;  // between two looks at the queues
+    // sweeps between two looks at the queues; the loop over them spills at K = 4 and with the 80
+    // registers of the exact 16-row tile (1.27 against 1.19 ms at 512 x 512 x 256)
+    constexpr int kSweeps = K <= 3 && (FAST || S::THREADS <= 512) ? 2 : 1;
     constexpr int kVec = (3 * K + 4) / 4;    // 16-byte words of an entry in use
     using F = std::conditional_t<kSlots == 2, float2, float>;
     const int lane = threadIdx.x & 31;

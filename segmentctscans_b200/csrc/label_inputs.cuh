@@ -102,7 +102,7 @@ int grad_magn_tiled(potts_context *ctx, const Geometry &g, const float *d_u, flo
     }
     POTTS_TRY(plan_tiles(ctx, g.ns, TileChoice{T::TR, T::TN, 1, ctx->gm_segment}));
     if (ctx->n_work == 0) return POTTS_OK;
-    POTTS_TRY(ensure(ctx, ctx->err, sizeof(int)));
+    POTTS_TRY(ensure(ctx, ctx->err, kErrBytes));
     CUtensorMap map;
     const uint64_t dims[2] = {(uint64_t)g.nstride_w, (uint64_t)g.n_lines};
     const uint64_t strides[1] = {sizeof(float) * (uint64_t)g.nstride_w};

@@ -201,6 +201,10 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// A context's error word and tv_range_kernel's flag.  Always both: a batch's captured graphs hold the
+// buffer's address, so no later call may have to grow it.
+constexpr size_t kErrBytes = 2 * sizeof(int);
+
 // Device buffers of a finished tape, kept by its context for the next one: allocating and freeing
 // several GB costs more than a tenth of a forward and backward pass (192^3, 40 iterations: 9 of 47 ms).
 // Bounded: the buffers of one tape, at most kTapePoolBytes.  Given back when the context is destroyed
@@ -1062,7 +1066,7 @@ int solve_k(potts_context *ctx, const float *d_u, const float *ci, float lam, fl
     ctx->seg_used = 0;
     ctx->seg_open = false;
     ctx->loop_launches = ctx->total_launches = ctx->loop_iters = 0;
-    POTTS_TRY(ensure(ctx, ctx->err, sizeof(int)));
+    POTTS_TRY(ensure(ctx, ctx->err, kErrBytes));
     POTTS_CUDA(cudaMemsetAsync(ctx->err.p, 0, sizeof(int), ctx->stream));
     POTTS_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     for (int sl = 0; sl < n_slabs; ++sl) {
@@ -1260,7 +1264,7 @@ int tv_run(potts_context *ctx, float *d_g, float lam, float tau, int iters, int 
     const size_t planes = variant == POTTS_VARIANT_PLAIN ? 4 : 6;
     POTTS_TRY(ensure(ctx, ctx->state, sizeof(float) * planes * (size_t)std::max<int64_t>(g.plane_w, 1)));
     POTTS_TRY(ensure(ctx, ctx->dq, sizeof(float) * (size_t)std::max(iters, 1)));
-    POTTS_TRY(ensure(ctx, ctx->err, 2 * sizeof(int)));  // error word, tv_range_kernel's flag
+    POTTS_TRY(ensure(ctx, ctx->err, kErrBytes));  // error word, tv_range_kernel's flag
     float *xi = static_cast<float *>(ctx->state.p), *v = xi + 3 * g.plane_w;
     float *xi_b = xi + 3 * g.plane_w;  // fused forms: the second half
     float *dq = static_cast<float *>(ctx->dq.p);

@@ -388,7 +388,7 @@ int shard_solve_k(potts_shard *const *sh, int n, int iters, float *const *d_res,
     ctx->seg_used = 0;
     ctx->seg_open = false;
     ctx->loop_launches = ctx->total_launches = ctx->loop_iters = 0;
-    POTTS_TRY(ensure(ctx, ctx->err, sizeof(int)));
+    POTTS_TRY(ensure(ctx, ctx->err, kErrBytes));
     POTTS_CUDA(cudaMemsetAsync(ctx->err.p, 0, sizeof(int), st));
     POTTS_CUDA(cudaEventRecord(ctx->ev0, st));
     std::vector<Geometry> g(n), gown(n);

@@ -35,3 +35,21 @@ def test_context_rechooses_for_another_volume(cuda_device):
                 f = potts.solve_host(ctx, m, u, ci, 30.0, TAU, TAU, 6, arith=arith, stats=True)
                 p = potts.solve_host(ctx, m, u, ci, 30.0, TAU, TAU, 6, arith=arith, stats=True, variant=1)
                 np.testing.assert_array_equal(f.dq_trace, p.dq_trace)
+
+
+def test_batch_runs_again_after_other_calls_of_its_context(cuda_device):
+    """The captured graphs hold device addresses of the context: denoising and solves in between leave
+    them valid."""
+    import torch
+
+    m, u, ci = random_volume(*SIZES[1], 3, seed=3)
+    du, lab = torch.from_numpy(u).cuda(), torch.zeros(m.span, dtype=torch.uint8, device="cuda")
+    g = du.clone()
+    torch.cuda.synchronize()
+    with potts.make_context(0) as ctx:
+        with potts.Batch(ctx, [potts.BatchVolume(m, du.data_ptr(), ci, 30.0, labels_ptr=lab.data_ptr())], TAU, TAU,
+                         9) as b:
+            first = b.run().dq_trace.copy()
+            potts.tv_denoise(ctx, m, g.data_ptr(), 0.06, 0.16, 3)
+            potts.solve_host(ctx, m, u, ci, 30.0, TAU, TAU, 3, arith="fast")
+            np.testing.assert_array_equal(b.run().dq_trace, first)
