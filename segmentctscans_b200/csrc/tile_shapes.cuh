@@ -3,12 +3,14 @@
 // the exact and the fast arithmetic (fused_*.cu).  Options can name the first
 // `named` entries.  exact / fast: time per voxel of a full tile relative to the
 // best shape's (per cent), measured on a 448 x 448 x 256 core of radius 215 over
-// the iterations 2 to 24; best_tiling weighs a volume's ragged tiles with them.
+// the iterations 2 to 24; choose_tile weighs a volume's ragged tiles with them.
 // Best shapes per iteration: K = 3 FP32 exact 0.844 ms (8 x 128 x 4; 16 x 64 x 2 0.871,
-// but 15 % the faster one where few voxels run the projection loop, 0.89 against 1.05 ms
-// at 4 % of them on 512 x 512 x 256: its weight is between), fast 0.593, bf16 0.882 and 0.605; K = 4 1.36 and 0.978; K = 5 2.09 and 1.24; K = 2 (512 x 512 x 256,
-// iterations 2 to 40, 8 x 64 x 4 with two blocks per multiprocessor) 0.589 and 0.452.  A K = 3 tile of
-// 8 x 64 x 4 with two blocks measured 0.840 against 0.806 ms fast and 1.33 against 1.17 exact there.
+// but 15 % faster where few voxels run the projection loop, 0.89 against 1.05 ms
+// at 4 % of them on 512 x 512 x 256: its weight is below), fast 0.593, bf16 0.882
+// and 0.605; K = 4 1.36 and 0.978; K = 5 2.09 and 1.24; K = 2 (512 x 512 x 256,
+// iterations 2 to 40, 8 x 64 x 4 with two blocks per multiprocessor) 0.589 and
+// 0.452.  A K = 3 tile of 8 x 64 x 4 with two blocks measured 0.840 against 0.806
+// ms fast and 1.33 against 1.17 exact there.
 #pragma once
 
 namespace potts {
