@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(kPlainThreads)
     __shared__ LoopList<3 * K + 3 * (K - 1)> list;
     if (threadIdx.x == 0) list.count = 0;
     __syncthreads();
+    int n = 0;  // entries in the list
     auto store = [&](int64_t o, const float (&pb)[K][3]) {
 #pragma unroll
         for (int i = 0; i < K - 1; ++i)
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(kPlainThreads)
             for (int j = 0; j < 3 * (K - 1); ++j) list.v[3 * K + j][e] = yb[j / 3][j % 3];
             list.off[e] = o;
         }
-        list.flush(c + 1 == kLoopChunks, [&](int i) {
+        list.flush(n, need, c + 1 == kLoopChunks, [&](int i) {
 #pragma unroll
             for (int j = 0; j < 3 * K; ++j) pq[j / 3][j % 3] = list.v[j][i];
 #pragma unroll

@@ -8,6 +8,7 @@
 
 #include <type_traits>
 
+#include "block.cuh"
 #include "geometry.cuh"
 #include "storage.cuh"
 #include "voxel.cuh"
@@ -15,8 +16,6 @@
 #include "voxel_fast.cuh"
 
 namespace potts {
-
-constexpr int kPlainThreads = 256;
 
 // Thread -> (line, n) for the split kernels: blocks walk the lines, each
 // block covers kPlainThreads consecutive n of one line.
@@ -58,42 +57,6 @@ __global__ void __launch_bounds__(kPlainThreads) init_kernel(Geometry g, const f
         if (Vb) Vb[i * g.plane_w + o] = Store<ST>::st(one);
     }
 }
-
-// The voxels of a block that need the projection loop: N floats each and the offset, column by
-// column (threads of a warp write and read different banks).  A block walks kLoopChunks chunks of
-// kPlainThreads voxels and runs the list when the next chunk might not fit (kCap entries, in 40 KB)
-// and at its end.
-constexpr int kLoopChunks = 4;
-template <int N>
-struct LoopList {
-    static constexpr int kCap = (N + 2) * 4 * 512 <= 40 * 1024 ? 512 : 256;
-    int64_t off[kCap];
-    float v[N][kCap];
-    int count;
-
-    // The entry of this thread's voxel (need: it has one); every thread of a warp calls it.
-    __device__ __forceinline__ int add(bool need)
-    {
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        const int lane = threadIdx.x & 31;
-        int first = 0;
-        if (lane == 0 && m) first = atomicAdd(&count, __popc(m));
-        return __shfl_sync(0xffffffffu, first, 0) + __popc(m & ((1u << lane) - 1u));
-    }
-    // run(i) for every entry when the list is to be emptied; every thread of the block calls it
-    // after each chunk.
-    template <typename Run>
-    __device__ __forceinline__ void flush(bool last, Run run)
-    {
-        __syncthreads();
-        const int n = count;
-        if (!last && n <= kCap - kPlainThreads) return;  // the same in every thread
-        for (int i = (int)threadIdx.x; i < n; i += kPlainThreads) run(i);
-        __syncthreads();
-        if (threadIdx.x == 0) count = 0;
-        __syncthreads();
-    }
-};
 
 // What the dual step reads at one voxel (missing neighbours as zeros).
 template <int K, typename ST>
@@ -155,6 +118,7 @@ __global__ void __launch_bounds__(kPlainThreads) dual_kernel(Geometry g, ST *__r
         __shared__ LoopList<3 * K> list;
         if (threadIdx.x == 0) list.count = 0;
         __syncthreads();
+        int n = 0;  // entries in the list
         float q[K][3];
         auto store = [&](int64_t o) {
             float xo[3 * (K - 1)];
@@ -186,7 +150,7 @@ __global__ void __launch_bounds__(kPlainThreads) dual_kernel(Geometry g, ST *__r
                 for (int j = 0; j < 3 * K; ++j) list.v[j][e] = q[j / 3][j % 3];
                 list.off[e] = o;
             }
-            list.flush(c + 1 == kLoopChunks, [&](int i) {
+            list.flush(n, need, c + 1 == kLoopChunks, [&](int i) {
 #pragma unroll
                 for (int j = 0; j < 3 * K; ++j) q[j / 3][j % 3] = list.v[j][i];
                 if constexpr (FAST)
