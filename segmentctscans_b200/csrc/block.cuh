@@ -8,6 +8,11 @@ namespace potts {
 
 constexpr int kPlainThreads = 256;
 
+// A barrier of the block, and whether a wait of any thread had given up before it: the same answer in
+// every thread.  (Read behind the barrier, the flag may already be set by a warp that has gone on to its
+// next wait, and the warps leave their loop at different barriers.)
+__device__ __forceinline__ bool sync_aborted(const volatile int *abort) { return __syncthreads_or(*abort) != 0; }
+
 // The voxels of a block that need the projection loop: N floats each and the offset, column by
 // column (threads of a warp write and read different banks).  A block walks kLoopChunks chunks of
 // kPlainThreads voxels and runs the list when the next chunk might not fit (kCap entries, in 40 KB)

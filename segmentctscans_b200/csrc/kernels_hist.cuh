@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "block.cuh"
 #include "geometry.cuh"
 #include "tma.cuh"
 
@@ -301,8 +302,7 @@ __global__ void __launch_bounds__(kGmThreads, kGmBlocks)
     for (int c = ca; c < cb; ++c) {
         wait_plane(c + 1);
         // past this barrier every thread is done with plane c-2: its slot takes plane c+SLOTS-2
-        __syncthreads();
-        if (*abort) break;
+        if (sync_aborted(abort)) break;
         if (t == 0 && c + T::SLOTS - 2 <= cb) issue(c + T::SLOTS - 2);
         const int4 ci = col_at(c), cp = col_at(c - 1), cn = col_at(c + 1);
         const float *X = smf + slot_of(c) * T::SLOT;

@@ -12,6 +12,7 @@
 
 #include <cstdint>
 
+#include "block.cuh"
 #include "geometry.cuh"
 #include "kernels_plain.cuh"
 #include "tma.cuh"
@@ -462,8 +463,7 @@ __global__ void __launch_bounds__(kTvThreads, kTvBlocks)
             }
         }
         // past this barrier every warp is done with plane c's xi slot and v slot
-        __syncthreads();
-        if (__shfl_sync(0xffffffffu, *abort, 0)) break;
+        if (sync_aborted(abort)) break;
         if (t == 0 && c + 3 <= cb) issue(c + 3, sc);
         v = vn;
         gc = gn, ge = gne, gn = g2, gne = g2e, gd = gd1;

@@ -46,6 +46,7 @@ unsigned wait_at(At at, unsigned in, int src)
 }
 void __syncthreads() { wait_at(At::kBarrier, 0, 0); }
 int __syncthreads_count(int p) { return (int)wait_at(At::kBarrier, p != 0, 0); }
+int __syncthreads_or(int p) { return wait_at(At::kBarrier, p != 0, 0) != 0; }
 unsigned __ballot_sync(unsigned, int p) { return wait_at(At::kWarp, p != 0, -1); }
 int __shfl_sync(unsigned, int v, int src) { return (int)wait_at(At::kWarp, (unsigned)v, src); }
 int __popc(unsigned v) { return __builtin_popcount(v); }
@@ -179,6 +180,36 @@ bool check_list(const std::vector<int> &rank, std::mt19937 &rng)
     return true;
 }
 
+// ---- sync_aborted: when one warp's wait gives up, all leave the loop after the same pass
+volatile int abort_flag = 0;
+int give_up_warp = 0, give_up_pass = 0;
+std::vector<int> passes;
+
+void abort_kernel()
+{
+    if (threadIdx.x == 0) abort_flag = 0;
+    __syncthreads();
+    int pass = 0;
+    for (; pass < 6; ++pass) {
+        if ((int)threadIdx.x / 32 == give_up_warp && pass == give_up_pass) abort_flag = 1;
+        if (potts::sync_aborted(&abort_flag)) break;
+    }
+    passes[threadIdx.x] = pass;
+    __syncthreads();
+}
+
+bool check_abort(const std::vector<int> &rank)
+{
+    for (give_up_warp = 0; give_up_warp < kThreads / 32; ++give_up_warp)
+        for (give_up_pass = 0; give_up_pass <= 6; ++give_up_pass) {  // 6: none
+            passes.assign((size_t)kThreads, -1);
+            if (!run_block(abort_kernel, rank)) return false;
+            for (int p : passes)
+                if (p != give_up_pass) return false;
+        }
+    return true;
+}
+
 }  // namespace
 
 int main()
@@ -207,5 +238,8 @@ int main()
             bad += !check_list<6>(r, rng) + !check_list<18>(r, rng) + !check_list<21>(r, rng) + !check_list<33>(r, rng);
         }
     std::printf("loop list: %d of %zu runs wrong\n", bad, sizeof(shares) / sizeof(shares[0]) * ranks.size() * 4);
-    return bad != 0;
+    int apart = 0;
+    for (const auto &r : ranks) apart += !check_abort(r);
+    std::printf("abort: %d of %zu orders wrong\n", apart, ranks.size());
+    return bad + apart != 0;
 }

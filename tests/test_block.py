@@ -1,6 +1,7 @@
 """What the threads of a block agree on (segmentctscans_b200/csrc/block.cuh), run on the host with the
 threads as coroutines in unfavourable orders (tests/cpp/block_check.cpp): the list of loop voxels runs
-every voxel once, with its own values, and its barriers pair up."""
+every voxel once, with its own values, and its barriers pair up; when a wait gives up, all threads leave
+their loop together."""
 import shutil
 import subprocess
 from pathlib import Path
