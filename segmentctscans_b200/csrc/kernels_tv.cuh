@@ -237,9 +237,9 @@ __device__ __forceinline__ float rcp_1ulp(float b)  // 1 / b, b normal
 }
 
 // xi <- (xi + tau G) / (1 + tau |G|) for four voxels; returns |dxi|^2 of each.  With 0 <= tau <= 1
-// (tau_in_range), |G|^2 <= 2^40 and no tiny numerators the root and the quotients are those of shrink_rn:
-// |G|^2 below 2^-80 gives a denominator of 1 whatever its root, so it is raised to that.  Else the IEEE
-// operations run (the same bits).
+// (tau_in_range), |G|^2 <= 2^40 (which a NaN is not) and no tiny numerators the root and the quotients
+// are those of shrink_rn: |G|^2 below 2^-80 gives a denominator of 1 whatever its root, so it is raised
+// to that.  Else the IEEE operations run (the same bits).
 __device__ __forceinline__ uint32_t below_key(float2 a)  // none_below_2m60's key of two values
 {
     const uint32_t x = __float_as_uint(a.x), y = __float_as_uint(a.y);
@@ -259,8 +259,8 @@ __device__ __forceinline__ Quad tv_step(Quad (&x)[3], const Quad (&G)[3], float 
     }
     const uint32_t key = min(min(min(below_key(a[0][0]), below_key(a[0][1])), min(below_key(a[0][2]), below_key(a[1][0]))),
                              min(below_key(a[1][1]), below_key(a[1][2])));
-    const float most = fmaxf(fmaxf(s[0].x, s[0].y), fmaxf(s[1].x, s[1].y));
-    if (tau_in_range && most <= 0x1p40f && key >= (67u << 24) - 1u) {
+    const float2 sum = add2(s[0], s[1]);  // not below any of the four; a NaN or infinite one makes it so
+    if (tau_in_range && sum.x + sum.y <= 0x1p40f && key >= (67u << 24) - 1u) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float2 mz;
