@@ -154,8 +154,12 @@ int potts_context_synchronize(potts_context *ctx);
 /* Kernel launches of the library on this context since the last solve began (a solve restarts the
  * count; the other calls add theirs); 0 for NULL.  No counterpart in the reference. */
 long long potts_context_launches(const potts_context *ctx);
-/* device_memory() (cuda-context/cuda-context.cpp:22-42): free bytes + bytes cached by this context. */
+/* device_memory() (cuda-context/cuda-context.cpp:22-42): free bytes + bytes that this context caches or that
+ * are kept of a closed tape. */
 int potts_device_memory(potts_context *ctx, size_t *available, size_t *total);
+/* Frees what is kept of a closed tape on the context's device (see potts_tape_destroy); for callers that
+ * share the device with another allocator. */
+int potts_context_trim(potts_context *ctx);
 
 /* DeviceField(mapping, stream, mr) (device-field-impl.h:24-33): uninitialised voxels. */
 int potts_field_create(potts_context *ctx, const potts_mapping *map, potts_field **out);
@@ -318,6 +322,10 @@ int potts_forward_ckpt(potts_context *ctx, const potts_mapping *map, const float
                        const float *ci, float lambda, float tau1, float tau2, int iters, int ckpt_every, float eps,
                        float *d_V, double *loss, potts_tape **out);
 int potts_backward(potts_tape *tape, float *d_grad_u, double *grad_ci, double *grad_lambda);
+/* From any thread, also after the tape's context.  While the context lives, the tape's device buffers (at most 8
+ * GiB, and an eighth of the free memory; one tape's per device) are kept for the next tape.  The library gives
+ * them back when it needs memory and when the context is destroyed; to other allocators they are in use
+ * until then, or until potts_context_trim. */
 void potts_tape_destroy(potts_tape *tape);
 
 /* ---------------------------------------------------------------------------

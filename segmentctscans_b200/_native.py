@@ -101,6 +101,7 @@ SIGNATURES = {
     "potts_context_synchronize": (_I, [_P]),
     "potts_context_launches": (ctypes.c_longlong, [_P]),
     "potts_device_memory": (_I, [_P, ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)]),
+    "potts_context_trim": (_I, [_P]),
     "potts_field_create": (_I, [_P, _MP, ctypes.POINTER(_P)]),
     "potts_field_upload": (_I, [_P, _MP, _FP, ctypes.POINTER(_P)]),
     "potts_field_download": (_I, [_P, _P, _FP, _U64]),

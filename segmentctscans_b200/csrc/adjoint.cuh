@@ -9,8 +9,9 @@
 }  // namespace
 
 struct potts_tape {
-    potts_context *ctx = nullptr;
-    std::shared_ptr<TapePool> pool;  // of the context, which this tape may outlive
+    potts_context *ctx = nullptr;  // which this tape may outlive
+    int device = 0;
+    cudaEvent_t done = nullptr;  // behind the last call's work on the context's stream
     MappingCopy mc;
     Geometry g{};
     DevBuf lines, ckpt, seg, A, X, Q, P, grads, loss;
@@ -24,31 +25,27 @@ struct potts_tape {
 
 namespace {
 
-void tape_bufs(potts_tape *t, DevBuf *(&bufs)[kTapeBufs])
+std::array<DevBuf *, kTapeBufs> tape_bufs(potts_tape *t)
 {
-    DevBuf *const all[kTapeBufs] = {&t->lines, &t->ckpt, &t->seg, &t->A, &t->X, &t->Q, &t->P, &t->grads, &t->loss};
-    std::copy(all, all + kTapeBufs, bufs);
+    return {&t->lines, &t->ckpt, &t->seg, &t->A, &t->X, &t->Q, &t->P, &t->grads, &t->loss};
 }
 
-void tape_free(potts_tape *t)
+// keep: the next tape may have the buffers.
+void tape_free(potts_tape *t, bool keep)
 {
     if (!t) return;
-    if (t->pool && t->pool->open) {
-        cudaSetDevice(t->ctx->device);
-        cudaStreamSynchronize(t->ctx->stream);
+    cudaSetDevice(t->device);
+    if (t->done) {
+        cudaEventSynchronize(t->done);
+        cudaEventDestroy(t->done);
     }
-    DevBuf *bufs[kTapeBufs];
-    tape_bufs(t, bufs);
-    size_t bytes = 0;
-    for (DevBuf *d : bufs) bytes += d->bytes;
-    // kept in place of an earlier tape's (the stream is idle: nothing uses them)
-    if (t->pool && t->pool->open && bytes <= kTapePoolBytes) {
-        t->pool->give_back();
-        for (int i = 0; i < kTapeBufs; ++i) t->pool->buf[i] = *bufs[i];
-    } else {
-        for (DevBuf *d : bufs)
-            if (d->p) cudaFree(d->p);
-    }
+    TapeBufs bufs{};
+    const auto own = tape_bufs(t);
+    for (size_t i = 0; i < own.size(); ++i) bufs[i] = *own[i];
+    if (keep)
+        TapePool::of(t->device).put(t->ctx, bufs);
+    else
+        free_tape_bufs(bufs);
     delete t;
 }
 
@@ -183,40 +180,33 @@ int tape_backward(potts_tape *t, float *d_grad_u, double *grad_ci, double *grad_
     return POTTS_OK;
 }
 
+// The tape's buffers: a closed tape's where they fit, else new ones.
 int tape_alloc(potts_tape *t)
 {
     potts_context *ctx = t->ctx;
     const size_t state = sizeof(float) * tape_state_floats(t);
     const size_t pw = sizeof(float) * (size_t)t->g.plane_w;
-    // an earlier tape's buffers where each is large enough, and at most twice what is needed; else its
-    // memory is given back first
-    const size_t sizes[kTapeBufs] = {0, state * (size_t)t->n_ckpt, state * ((size_t)t->every + 1),
-                                     pw * (size_t)(t->K - 1), pw * 3 * (size_t)(t->K - 1), pw * (size_t)t->K,
-                                     pw * 3 * (size_t)t->K, 0, 0};
-    DevBuf *bufs[kTapeBufs];
-    tape_bufs(t, bufs);
-    bool fits = t->pool->bytes() > 0;
-    for (int i = 1; i < 7; ++i) {
-        const size_t have = t->pool->buf[i].bytes;
-        fits = fits && have >= sizes[i] && have / 2 <= sizes[i];
+    const size_t K = (size_t)t->K;
+    const size_t sizes[kTapeBufs] = {sizeof(int4) * (size_t)std::max<int64_t>(t->mc.n_lines, 1),
+                                     state * (size_t)t->n_ckpt,
+                                     state * ((size_t)t->every + 1),
+                                     pw * (K - 1),
+                                     pw * 3 * (K - 1),
+                                     pw * K,
+                                     pw * 3 * K,
+                                     sizeof(double) * (POTTS_MAX_PHASES + 1),
+                                     sizeof(double)};
+    const auto own = tape_bufs(t);
+    TapeBufs bufs{};
+    if (TapePool::of(t->device).take(sizes, bufs)) {
+        for (size_t i = 0; i < own.size(); ++i) *own[i] = bufs[i];
+    } else {
+        size_t need = size_t(256) << 20, free_b = 0;
+        for (size_t b : sizes) need += b;
+        POTTS_TRY(planning_memory(ctx, need, &free_b));
+        if (need > free_b) return fail(POTTS_ENOMEM, "the checkpoints and the segment's states do not fit in memory");
+        for (size_t i = 0; i < own.size(); ++i) POTTS_TRY(ensure(ctx, *own[i], sizes[i]));
     }
-    if (fits) {
-        for (int i = 1; i < kTapeBufs; ++i) std::swap(*bufs[i], t->pool->buf[i]);
-    }
-    t->pool->give_back();
-    size_t free_b = 0, total_b = 0;
-    POTTS_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const size_t need = fits ? 0 : state * ((size_t)t->n_ckpt + (size_t)t->every + 1) +
-                        pw * ((size_t)(t->K - 1) * 4 + (size_t)t->K * 4) + (size_t(256) << 20);
-    if (need > free_b) return fail(POTTS_ENOMEM, "the checkpoints and the segment's states do not fit in memory");
-    POTTS_TRY(ensure(ctx, t->ckpt, state * (size_t)t->n_ckpt));
-    POTTS_TRY(ensure(ctx, t->seg, state * ((size_t)t->every + 1)));
-    POTTS_TRY(ensure(ctx, t->A, pw * (size_t)(t->K - 1)));
-    POTTS_TRY(ensure(ctx, t->X, pw * 3 * (size_t)(t->K - 1)));
-    POTTS_TRY(ensure(ctx, t->Q, pw * (size_t)t->K));
-    POTTS_TRY(ensure(ctx, t->P, pw * 3 * (size_t)t->K));
-    POTTS_TRY(ensure(ctx, t->grads, sizeof(double) * (POTTS_MAX_PHASES + 1)));
-    POTTS_TRY(ensure(ctx, t->loss, sizeof(double)));
     // the kernels read (and multiply by 0) neighbours outside the mask
     POTTS_CUDA(cudaMemsetAsync(t->Q.p, 0, t->Q.bytes, ctx->stream));
     return POTTS_OK;

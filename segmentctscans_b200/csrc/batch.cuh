@@ -295,9 +295,8 @@ int batch_build(potts_batch *b)
             bv.voxels += (uint64_t)((m.base[c + 1] - m.base[c]) / m.nstride) * m.n_images;
         b->voxels += bv.voxels;
     }
-    size_t free_b = 0, total_b = 0;
-    ctx->tape_pool->give_back();
-    POTTS_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    size_t free_b = 0;
+    POTTS_TRY(planning_memory(ctx, state + (size_t(512) << 20), &free_b));
     if (state + (size_t(512) << 20) > free_b) return fail(POTTS_ENOMEM, "the batch's state does not fit in memory");
     b->state_bytes = state;
     POTTS_TRY(ensure(ctx, b->state, state));

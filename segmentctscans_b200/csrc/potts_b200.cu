@@ -205,30 +205,110 @@ struct DevBuf {
 // buffer's address, so no later call may have to grow it.
 constexpr size_t kErrBytes = 2 * sizeof(int);
 
-// Device buffers of a finished tape, kept by its context for the next one: allocating and freeing
-// several GB costs more than a tenth of a forward and backward pass (192^3, 40 iterations: 9 of 47 ms).
-// Bounded: the buffers of one tape, at most kTapePoolBytes.  Given back when the context is destroyed
-// and before the library plans a solve, a batch, a shard or a tape by the free memory, or when an
-// allocation fails.  A tape may outlive its context: it shares the pool, which is then closed.
+// Device buffers of the tape that was closed last on a device, kept for the next one of any context:
+// allocating and freeing several GB costs more than a tenth of a forward and backward pass (192^3, 40
+// iterations: 9 of 47 ms).  (The driver's own pools give memory back by themselves, but take 46 ms for the
+// first allocation of 6.7 GB and 73 ms for giving it back, where cudaMalloc and cudaFree take 3 and 8.)
+// Bounded: one tape's buffers per device, at most kTapePoolBytes and an eighth of the memory that is free
+// beside them.  Given back when the context of that tape is destroyed, before that context plans a solve, a
+// batch or a tape by the free memory, before any context of the device does so and finds too little, when
+// an allocation of the library fails, and by potts_context_trim.  Contexts of several threads share it, and a
+// tape may be closed by any thread, also after its context.
 constexpr int kTapeBufs = 9;
 constexpr size_t kTapePoolBytes = size_t(8) << 30;
-struct TapePool {
-    DevBuf buf[kTapeBufs];
-    bool open = true;
+using TapeBufs = std::array<DevBuf, kTapeBufs>;
 
-    size_t bytes() const
+size_t tape_bytes(const TapeBufs &bufs)
+{
+    size_t n = 0;
+    for (const DevBuf &b : bufs) n += b.bytes;
+    return n;
+}
+
+// (cudaFree waits for work on the device that may still use a buffer.)
+void free_tape_bufs(const TapeBufs &bufs)
+{
+    for (const DevBuf &b : bufs)
+        if (b.p) cudaFree(b.p);
+}
+
+class TapePool {
+public:
+    static TapePool &of(int device)
     {
-        size_t n = 0;
-        for (const DevBuf &b : buf) n += b.bytes;
-        return n;
+        // never destroyed: a context or a tape may be closed while the program's statics are
+        static std::vector<TapePool> *const pools = [] {
+            int n = 0;
+            if (cudaGetDeviceCount(&n) != cudaSuccess) n = 0;
+            return new std::vector<TapePool>((size_t)std::max(n, 1));
+        }();
+        return (*pools)[(size_t)device < pools->size() ? (size_t)device : 0];
     }
-    void give_back()
+
+    void add_context(const potts_context *ctx)
     {
-        for (DevBuf &b : buf) {
-            if (b.p) cudaFree(b.p);  // waits for work on the device that may still use it
-            b = DevBuf{};
+        std::lock_guard<std::mutex> lock(mtx_);
+        contexts_.push_back(ctx);
+    }
+    void remove_context(const potts_context *ctx)
+    {
+        {
+            std::lock_guard<std::mutex> lock(mtx_);
+            contexts_.erase(std::remove(contexts_.begin(), contexts_.end(), ctx), contexts_.end());
         }
+        give_back(ctx);
     }
+
+    size_t bytes()
+    {
+        std::lock_guard<std::mutex> lock(mtx_);
+        return tape_bytes(kept_);
+    }
+
+    // Moves the kept buffers into `bufs` if each is as large as sizes[i], and at most twice as large.
+    bool take(const size_t (&sizes)[kTapeBufs], TapeBufs &bufs)
+    {
+        std::lock_guard<std::mutex> lock(mtx_);
+        if (tape_bytes(kept_) == 0) return false;
+        for (int i = 0; i < kTapeBufs; ++i)
+            if (kept_[(size_t)i].bytes < sizes[i] || kept_[(size_t)i].bytes / 2 > sizes[i]) return false;
+        bufs = std::exchange(kept_, TapeBufs{});
+        return true;
+    }
+
+    // Keeps the buffers of a tape of `ctx` (nothing on the device uses them) in place of an earlier one's, or
+    // frees them.
+    void put(const potts_context *ctx, TapeBufs bufs)
+    {
+        size_t free_b = 0, total_b = 0;
+        const size_t bytes = tape_bytes(bufs);
+        if (bytes > 0 && bytes <= kTapePoolBytes && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+            bytes <= free_b / 8) {
+            std::lock_guard<std::mutex> lock(mtx_);
+            if (std::find(contexts_.begin(), contexts_.end(), ctx) != contexts_.end()) {
+                std::swap(kept_, bufs);
+                owner_ = ctx;
+            }
+        }
+        free_tape_bufs(bufs);
+    }
+
+    // Frees the kept buffers (with a context: if they are of a tape of that context).
+    void give_back(const potts_context *ctx = nullptr)
+    {
+        TapeBufs bufs{};
+        {
+            std::lock_guard<std::mutex> lock(mtx_);
+            if (!ctx || owner_ == ctx) std::swap(kept_, bufs);
+        }
+        free_tape_bufs(bufs);
+    }
+
+private:
+    std::mutex mtx_;
+    TapeBufs kept_{};
+    const potts_context *owner_ = nullptr;  // of the tape that the kept buffers were
+    std::vector<const potts_context *> contexts_;
 };
 
 }  // namespace
@@ -269,7 +349,6 @@ struct potts_context {
     int loop_iters = 0;  // iterations inside the event pairs
     // control words of persistent fused launches (item counters per iteration, grid barrier)
     DevBuf pctl;
-    std::shared_ptr<TapePool> tape_pool = std::make_shared<TapePool>();
 };
 
 struct potts_field {
@@ -328,7 +407,7 @@ int ensure(potts_context *ctx, DevBuf &b, size_t bytes)
     if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
-        ctx->tape_pool->give_back();
+        TapePool::of(ctx->device).give_back();
         POTTS_CUDA(cudaMalloc(&b.p, bytes));
     }
     b.bytes = bytes;
@@ -349,7 +428,23 @@ int release(potts_context *ctx, DevBuf &b)
 size_t cached_bytes(const potts_context *ctx)
 {
     return ctx->state.bytes + ctx->partial.bytes + ctx->host_u.bytes + ctx->host_res.bytes + ctx->host_labels.bytes +
-           ctx->ustage.bytes + ctx->hist.bytes + ctx->io.bytes + ctx->io_tables.bytes + ctx->tape_pool->bytes();
+           ctx->ustage.bytes + ctx->hist.bytes + ctx->io.bytes + ctx->io_tables.bytes;
+}
+
+// Free device memory for a plan that needs `need` bytes of it: a closed tape's buffers are given back first,
+// those of another context's tape only if the plan does not fit beside them (freeing waits for the whole
+// device).
+int planning_memory(potts_context *ctx, uint64_t need, size_t *free_b)
+{
+    TapePool &pool = TapePool::of(ctx->device);
+    size_t total_b = 0;
+    pool.give_back(ctx);
+    POTTS_CUDA(cudaMemGetInfo(free_b, &total_b));
+    if (need > *free_b && pool.bytes() > 0) {
+        pool.give_back();
+        POTTS_CUDA(cudaMemGetInfo(free_b, &total_b));
+    }
+    return POTTS_OK;
 }
 
 int upload_lines(potts_context *ctx, const potts_mapping *map)
@@ -1007,12 +1102,12 @@ int solve_k(potts_context *ctx, const float *d_u, const float *ci, float lam, fl
     // staging buffers are scratch of earlier calls: the solve gets their memory.
     POTTS_TRY(release(ctx, ctx->io));
     POTTS_TRY(release(ctx, ctx->io_tables));
-    ctx->tape_pool->give_back();
-    size_t free_b = 0, total_b = 0;
-    POTTS_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t margin = size_t(512) << 20;
-    const size_t avail = free_b + ctx->state.bytes > margin ? free_b + ctx->state.bytes - margin : 0;
     const uint64_t bytes_per_slice = sizeof(ST) * (uint64_t)planes * (uint64_t)std::max<int64_t>(mc.n_lines, 1);
+    const uint64_t whole = bytes_per_slice * get_stride((uint32_t)n) + margin;
+    size_t free_b = 0;
+    POTTS_TRY(planning_memory(ctx, whole - std::min<uint64_t>(whole, ctx->state.bytes), &free_b));
+    const size_t avail = free_b + ctx->state.bytes > margin ? free_b + ctx->state.bytes - margin : 0;
     int slab_w = o.slab_w > 0 ? o.slab_w : (int)std::min<uint64_t>(prev_stride(avail / bytes_per_slice), 0x7fffffe0u);
     const int halo = iters;
     int res_w = n, n_slabs = 1;
@@ -1197,6 +1292,7 @@ int context_init(int device, void *stream, bool use_stream, potts_context **out)
         potts_context_destroy(ctx);
         return fail(POTTS_ECUDA, "event/pinned allocation failed");
     }
+    TapePool::of(device).add_context(ctx);
     *out = ctx;
     return POTTS_OK;
 }
@@ -1405,8 +1501,7 @@ void potts_context_destroy(potts_context *ctx)
                       &ctx->host_res, &ctx->host_labels, &ctx->ustage, &ctx->err, &ctx->cols, &ctx->work, &ctx->vols,
                       &ctx->hist, &ctx->hist_aux, &ctx->range, &ctx->io, &ctx->io_tables, &ctx->pctl})
         if (b->p) cudaFree(b->p);
-    ctx->tape_pool->give_back();
-    ctx->tape_pool->open = false;
+    TapePool::of(ctx->device).remove_context(ctx);
     if (ctx->pinned_dq) cudaFreeHost(ctx->pinned_dq);
     for (cudaEvent_t e : ctx->seg_ev) cudaEventDestroy(e);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -1428,8 +1523,16 @@ int potts_device_memory(potts_context *ctx, size_t *available, size_t *total)
     POTTS_CUDA(cudaSetDevice(ctx->device));
     size_t f = 0, t = 0;
     POTTS_CUDA(cudaMemGetInfo(&f, &t));
-    *available = f + cached_bytes(ctx);
+    *available = f + cached_bytes(ctx) + TapePool::of(ctx->device).bytes();
     *total = t;
+    return POTTS_OK;
+}
+
+int potts_context_trim(potts_context *ctx)
+{
+    if (!ctx) return fail(POTTS_EINVAL, "context is NULL");
+    POTTS_CUDA(cudaSetDevice(ctx->device));
+    TapePool::of(ctx->device).give_back();
     return POTTS_OK;
 }
 
@@ -1447,9 +1550,9 @@ int potts_field_create(potts_context *ctx, const potts_mapping *map, potts_field
     cudaSetDevice(ctx->device);
     const size_t bytes = sizeof(float) * (size_t)std::max<uint64_t>(f->mapping.span, 1);
     cudaError_t e = cudaMalloc(&f->d, bytes);
-    if (e != cudaSuccess && ctx->tape_pool->bytes() > 0) {
+    if (e != cudaSuccess && TapePool::of(ctx->device).bytes() > 0) {
         cudaGetLastError();
-        ctx->tape_pool->give_back();
+        TapePool::of(ctx->device).give_back();
         e = cudaMalloc(&f->d, bytes);
     }
     if (e != cudaSuccess) {
@@ -1742,8 +1845,10 @@ int potts_forward_ckpt(potts_context *ctx, const potts_mapping *map, const float
     POTTS_CUDA(cudaSetDevice(ctx->device));
     auto *t = new potts_tape();
     t->ctx = ctx;
-    t->pool = ctx->tape_pool;
+    t->device = ctx->device;
     int rc = copy_mapping(map, t->mc);
+    if (rc == POTTS_OK && cudaEventCreateWithFlags(&t->done, cudaEventDisableTiming) != cudaSuccess)
+        rc = fail(POTTS_ECUDA, "cudaEventCreate failed");
     if (rc == POTTS_OK) {
         t->K = K;
         t->iters = iters;
@@ -1765,14 +1870,13 @@ int potts_forward_ckpt(potts_context *ctx, const potts_mapping *map, const float
         t->g.slab_start = 0;
         uint64_t vox = (uint64_t)t->mc.n_lines * m.n_images;
         t->inv_count = vox > 0 ? 1.0 / (double)vox : 0.0;
-        rc = ensure(ctx, t->lines, sizeof(int4) * (size_t)std::max<int64_t>(t->mc.n_lines, 1));
+        rc = tape_alloc(t);
         if (rc == POTTS_OK && t->mc.n_lines > 0 &&
-            cudaMemcpy(t->lines.p, t->mc.lines.data(), sizeof(int4) * t->mc.n_lines, cudaMemcpyHostToDevice) !=
-                cudaSuccess)
+            cudaMemcpyAsync(t->lines.p, t->mc.lines.data(), sizeof(int4) * t->mc.n_lines, cudaMemcpyHostToDevice,
+                            ctx->stream) != cudaSuccess)
             rc = fail(POTTS_ECUDA, "copying the line table failed");
         t->g.lines = static_cast<const int4 *>(t->lines.p);
     }
-    if (rc == POTTS_OK) rc = tape_alloc(t);
     if (rc == POTTS_OK && t->mc.n_lines > 0) {
         switch (K) {
         case 2: rc = tape_forward<2>(t, d_V, loss); break;
@@ -1784,9 +1888,10 @@ int potts_forward_ckpt(potts_context *ctx, const potts_mapping *map, const float
     } else if (rc == POTTS_OK && loss) {
         *loss = 0.0;
     }
+    if (t->done) cudaEventRecord(t->done, ctx->stream);
     if (rc != POTTS_OK) {
         const std::string msg = g_last_error;
-        tape_free(t);
+        tape_free(t, false);
         g_last_error = msg;
         return rc;
     }
@@ -1804,17 +1909,19 @@ int potts_backward(potts_tape *t, float *d_grad_u, double *grad_ci, double *grad
             for (int i = 0; i < t->K; ++i) grad_ci[i] = 0.0;
         return POTTS_OK;
     }
+    int rc = fail(POTTS_EINVAL, "K must be in [2, 6]");
     switch (t->K) {
-    case 2: return tape_backward<2>(t, d_grad_u, grad_ci, grad_lambda);
-    case 3: return tape_backward<3>(t, d_grad_u, grad_ci, grad_lambda);
-    case 4: return tape_backward<4>(t, d_grad_u, grad_ci, grad_lambda);
-    case 5: return tape_backward<5>(t, d_grad_u, grad_ci, grad_lambda);
-    case 6: return tape_backward<6>(t, d_grad_u, grad_ci, grad_lambda);
+    case 2: rc = tape_backward<2>(t, d_grad_u, grad_ci, grad_lambda); break;
+    case 3: rc = tape_backward<3>(t, d_grad_u, grad_ci, grad_lambda); break;
+    case 4: rc = tape_backward<4>(t, d_grad_u, grad_ci, grad_lambda); break;
+    case 5: rc = tape_backward<5>(t, d_grad_u, grad_ci, grad_lambda); break;
+    case 6: rc = tape_backward<6>(t, d_grad_u, grad_ci, grad_lambda); break;
     }
-    return fail(POTTS_EINVAL, "K must be in [2, 6]");
+    cudaEventRecord(t->done, t->ctx->stream);
+    return rc;
 }
 
-void potts_tape_destroy(potts_tape *t) { tape_free(t); }
+void potts_tape_destroy(potts_tape *t) { tape_free(t, true); }
 
 
 int potts_tv_denoise(potts_context *ctx, const potts_mapping *map, float *d_g, float lambda, float tau, int iters,

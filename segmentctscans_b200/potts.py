@@ -58,6 +58,10 @@ class CudaContext:
         check(_native.host_lib().potts_device_memory(self.handle, ctypes.byref(a), ctypes.byref(t)))
         return int(a.value), int(t.value)
 
+    def trim(self) -> None:
+        """Frees the device buffers that are kept of a closed Tape (potts_context_trim)."""
+        check(_native.host_lib().potts_context_trim(self.handle))
+
     def close(self) -> None:
         if self._h is not None:
             _native.host_lib().potts_context_destroy(self._h)
