@@ -433,14 +433,19 @@ size_t cached_bytes(const potts_context *ctx)
 
 // Free device memory for a plan that needs `need` bytes of it: a closed tape's buffers are given back first,
 // those of another context's tape only if the plan does not fit beside them (freeing waits for the whole
-// device).
+// device).  Under stream capture, where nothing can be freed, they stay.
 int planning_memory(potts_context *ctx, uint64_t need, size_t *free_b)
 {
     TapePool &pool = TapePool::of(ctx->device);
     size_t total_b = 0;
-    pool.give_back(ctx);
+    bool may_free = false;
+    if (pool.bytes() > 0) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        may_free = cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+        if (may_free) pool.give_back(ctx);
+    }
     POTTS_CUDA(cudaMemGetInfo(free_b, &total_b));
-    if (need > *free_b && pool.bytes() > 0) {
+    if (may_free && need > *free_b && pool.bytes() > 0) {
         pool.give_back();
         POTTS_CUDA(cudaMemGetInfo(free_b, &total_b));
     }

@@ -1,5 +1,5 @@
 """The device buffers that are kept of a closed tape: bounded by what is free, given back to whoever in the
-process asks through the library, and safe with several threads."""
+process asks through the library, safe with several threads, and not touched under stream capture."""
 import queue
 import threading
 
@@ -123,3 +123,32 @@ def test_threads_close_each_other_s_tapes(cuda_device):
         t.join(180)
     assert not any(t.is_alive() for t in threads) and not errors, errors
     assert abs(free_bytes() - before) < 64 * MB
+
+
+def test_a_captured_solve_leaves_the_kept_buffers(cuda_device):
+    """Nothing can be freed while a stream is captured: a split solve on a planned mapping is captured and
+    replayed with a closed tape's buffers in place."""
+    import torch
+
+    a = Inputs(volume(24, 22, 3, 1))
+    lab = torch.zeros(a.m.span, dtype=torch.uint8, device="cuda")
+    side = torch.cuda.Stream()
+
+    def solve(ctx):
+        potts.solve_device(ctx, a.m, a.u.data_ptr(), a.ci, 30.0, TAU, TAU, 6, labels_ptr=lab.data_ptr(), variant=1,
+                           track_dq=0, stats=False)
+
+    with potts.make_context(0, stream=side.cuda_stream) as ctx:
+        solve(ctx)
+        side.synchronize()
+        want = lab.clone()
+        a.tape(ctx).close()
+        lab.zero_()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            solve(ctx)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(lab, want)
+        del graph
