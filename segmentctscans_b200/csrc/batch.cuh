@@ -114,12 +114,9 @@ int batch_plan_tiles(potts_batch *b, const TileChoice &tile)
     POTTS_TRY(ensure(ctx, b->work_vol, sizeof(int) * std::max<size_t>(work.size(), 1)));
     POTTS_TRY(ensure(ctx, b->desc, sizeof(potts::FusedVolume<K, ST>) * desc.size()));
     POTTS_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (!work.empty()) {
-        POTTS_CUDA(cudaMemcpy(b->work.p, work.data(), sizeof(int4) * work.size(), cudaMemcpyHostToDevice));
-        POTTS_CUDA(cudaMemcpy(b->work_vol.p, work_vol.data(), sizeof(int) * work.size(), cudaMemcpyHostToDevice));
-    }
-    POTTS_CUDA(cudaMemcpy(b->desc.p, desc.data(), sizeof(potts::FusedVolume<K, ST>) * desc.size(),
-                          cudaMemcpyHostToDevice));
+    POTTS_TRY(upload_table(ctx, b->work.p, work, work.size()));
+    POTTS_TRY(upload_table(ctx, b->work_vol.p, work_vol, work.size()));
+    POTTS_TRY(upload_table(ctx, b->desc.p, desc, desc.size()));
     b->n_work = (int)work.size();
     b->tile = tile;
     return POTTS_OK;
@@ -308,12 +305,10 @@ int batch_build(potts_batch *b)
     POTTS_TRY(ensure(ctx, ctx->err, kErrBytes));
     for (BatchVolume &bv : b->vols) {
         int4 *dl = static_cast<int4 *>(b->lines.p) + bv.lines_off;
-        if (bv.mc.n_lines > 0)
-            POTTS_CUDA(cudaMemcpy(dl, bv.mc.lines.data(), sizeof(int4) * bv.mc.n_lines, cudaMemcpyHostToDevice));
+        POTTS_TRY(upload_table(ctx, dl, bv.mc.lines, (size_t)bv.mc.n_lines));
         bv.g.lines = dl;
         const std::vector<int4> cols = column_table(bv.mc.m);
-        POTTS_CUDA(cudaMemcpy(static_cast<int4 *>(b->cols.p) + bv.cols_off, cols.data(), sizeof(int4) * cols.size(),
-                              cudaMemcpyHostToDevice));
+        POTTS_TRY(upload_table(ctx, static_cast<int4 *>(b->cols.p) + bv.cols_off, cols, cols.size()));
     }
 
     // tile shape: the options', or the autotuner's

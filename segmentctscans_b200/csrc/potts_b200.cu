@@ -771,6 +771,16 @@ std::vector<int4> work_items(const potts_mapping &m, int ns, const TileChoice &t
     return work;
 }
 
+// Host tables to device memory in the order of the context's stream: a table that earlier calls' kernels may
+// still be reading is overwritten behind them.  (cudaMemcpy orders itself by the default stream only; the
+// pageable source is staged before this returns.)
+template <typename T>
+int upload_table(potts_context *ctx, void *dst, const std::vector<T> &src, size_t n)
+{
+    if (n > 0) POTTS_CUDA(cudaMemcpyAsync(dst, src.data(), sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream));
+    return POTTS_OK;
+}
+
 // Column table and work items of the context's mapping on the device.
 int plan_tiles(potts_context *ctx, int ns, const TileChoice &tc)
 {
@@ -778,15 +788,14 @@ int plan_tiles(potts_context *ctx, int ns, const TileChoice &tc)
     if (!ctx->cols_valid) {
         const std::vector<int4> cols = column_table(mc.m);
         POTTS_TRY(ensure(ctx, ctx->cols, sizeof(int4) * cols.size()));
-        POTTS_CUDA(cudaMemcpy(ctx->cols.p, cols.data(), sizeof(int4) * cols.size(), cudaMemcpyHostToDevice));
+        POTTS_TRY(upload_table(ctx, ctx->cols.p, cols, cols.size()));
         ctx->cols_valid = true;
     }
     const int key[5] = {ns, tc.rows, tc.slices, tc.segment, (int)mc.n_lines};
     if (std::equal(key, key + 5, ctx->work_key)) return POTTS_OK;
     const std::vector<int4> work = work_items(mc.m, ns, tc);
     POTTS_TRY(ensure(ctx, ctx->work, sizeof(int4) * std::max<size_t>(work.size(), 1)));
-    if (!work.empty())
-        POTTS_CUDA(cudaMemcpy(ctx->work.p, work.data(), sizeof(int4) * work.size(), cudaMemcpyHostToDevice));
+    POTTS_TRY(upload_table(ctx, ctx->work.p, work, work.size()));
     std::copy(key, key + 5, ctx->work_key);
     ctx->n_work = (int)work.size();
     return POTTS_OK;
@@ -1876,10 +1885,7 @@ int potts_forward_ckpt(potts_context *ctx, const potts_mapping *map, const float
         uint64_t vox = (uint64_t)t->mc.n_lines * m.n_images;
         t->inv_count = vox > 0 ? 1.0 / (double)vox : 0.0;
         rc = tape_alloc(t);
-        if (rc == POTTS_OK && t->mc.n_lines > 0 &&
-            cudaMemcpyAsync(t->lines.p, t->mc.lines.data(), sizeof(int4) * t->mc.n_lines, cudaMemcpyHostToDevice,
-                            ctx->stream) != cudaSuccess)
-            rc = fail(POTTS_ECUDA, "copying the line table failed");
+        if (rc == POTTS_OK) rc = upload_table(ctx, t->lines.p, t->mc.lines, (size_t)t->mc.n_lines);
         t->g.lines = static_cast<const int4 *>(t->lines.p);
     }
     if (rc == POTTS_OK && t->mc.n_lines > 0) {

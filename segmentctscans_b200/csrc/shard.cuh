@@ -272,11 +272,10 @@ int shard_create(potts_context *ctx, const potts_mapping *map, const uint32_t *c
     s->own_line_end = l1;
     const int64_t n_lines = s->mc.n_lines;
     POTTS_TRY(ensure(ctx, s->lines, sizeof(int4) * (size_t)std::max<int64_t>(n_lines, 1)));
-    if (n_lines > 0)
-        POTTS_CUDA(cudaMemcpy(s->lines.p, s->mc.lines.data(), sizeof(int4) * n_lines, cudaMemcpyHostToDevice));
+    POTTS_TRY(upload_table(ctx, s->lines.p, s->mc.lines, (size_t)n_lines));
     const std::vector<int4> cols = column_table(s->mc.m);
     POTTS_TRY(ensure(ctx, s->cols, sizeof(int4) * cols.size()));
-    POTTS_CUDA(cudaMemcpy(s->cols.p, cols.data(), sizeof(int4) * cols.size(), cudaMemcpyHostToDevice));
+    POTTS_TRY(upload_table(ctx, s->cols.p, cols, cols.size()));
     // tile and work items: the owned columns and, with a right neighbour, its first column
     // (the primal step there gives Vbar and V at b; see the top of this file)
     const uint32_t a = shard_local_col(s.get(), sc.own_begin);
@@ -289,8 +288,7 @@ int shard_create(potts_context *ctx, const potts_mapping *map, const uint32_t *c
     }
     const std::vector<int4> work = work_items(s->mc.m, (int)lm.n_images, s->tile, (int)a, (int)b1);
     POTTS_TRY(ensure(ctx, s->work, sizeof(int4) * std::max<size_t>(work.size(), 1)));
-    if (!work.empty())
-        POTTS_CUDA(cudaMemcpy(s->work.p, work.data(), sizeof(int4) * work.size(), cudaMemcpyHostToDevice));
+    POTTS_TRY(upload_table(ctx, s->work.p, work, work.size()));
     s->n_work = (int)work.size();
     const Geometry g = shard_geometry(s.get());
     s->state_bytes = store_bytes(o.storage) * 8 * (size_t)(K - 1) * (size_t)std::max<int64_t>(g.plane_w, 1);
