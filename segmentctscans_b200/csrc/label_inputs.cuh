@@ -96,7 +96,7 @@ int grad_magn_tiled(potts_context *ctx, const Geometry &g, const float *d_u, flo
     // the column segment is chosen once per mapping and slice count
     if (ctx->gm_segment == 0 || ctx->gm_ns != g.ns) {
         const potts_mapping &m = ctx->mapping.m;
-        march_time({{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, T::TR, T::TN,
+        march_time(march_runs({{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, T::TR), T::TN,
                    potts::kGmBlocks * std::max(ctx->n_sm, 1), 0, &ctx->gm_segment);
         ctx->gm_ns = g.ns;
     }

@@ -13,7 +13,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <functional>
 #include <type_traits>
 #include <utility>
 #include <string>
@@ -25,6 +24,7 @@
 #include "kernels_adjoint.cuh"
 #include "kernels_tiled.cuh"
 #include "tile_shapes.cuh"
+#include "march_plan.cuh"
 #include "kernels_hist.cuh"
 #include "kernels_tv.cuh"
 #include "kernels_fieldio.cuh"
@@ -585,108 +585,6 @@ int encode_map(CUtensorMap *m, CUtensorMapDataType dt, const void *base, int ran
 // (none: prefetching 2 or 4 planes measured 0.5-3 % slower at 768^2 x 1024).
 constexpr int kDefaultPrefetch = 0;
 
-// The slices and columns that a column-march kernel runs over.
-struct MarchVolume {
-    const potts_mapping *map;
-    int ns;
-    int c_begin, c_end;
-};
-
-// Columns [first, second) of a run of columns that hold a tile's rows.
-using ColumnRun = std::pair<int, int>;
-
-std::vector<ColumnRun> tile_runs(const potts_mapping &m, int r0, int rows, int c_begin, int c_end)
-{
-    std::vector<ColumnRun> runs;
-    for (int c = c_begin; c < c_end; ++c) {
-        const int64_t cnt = (int64_t)(m.base[c + 1] - m.base[c]) / m.nstride;
-        if (cnt <= 0 || (int64_t)m.start_row[c] >= r0 + rows || (int64_t)m.start_row[c] + cnt <= r0) continue;
-        if (!runs.empty() && runs.back().second == c)
-            runs.back().second = c + 1;
-        else
-            runs.push_back({c, c + 1});
-    }
-    return runs;
-}
-
-// First row and one past the last row of the columns [c_begin, c_end).
-std::pair<int, int> row_range(const potts_mapping &m, int c_begin, int c_end)
-{
-    int lo = INT32_MAX, hi = 0;
-    for (int c = c_begin; c < c_end; ++c) {
-        const int64_t cnt = (int64_t)(m.base[c + 1] - m.base[c]) / m.nstride;
-        if (cnt <= 0) continue;
-        lo = std::min<int>(lo, (int)m.start_row[c]);
-        hi = std::max<int>(hi, (int)(m.start_row[c] + cnt));
-    }
-    return {lo, hi};
-}
-
-// Column planes that a work item costs besides those of its columns: the plane
-// before and after them, filling the load ring and the drain at its end.  With
-// 4 the choice below was within 2 % (at most 9 %) of the best of 13 segment
-// lengths on cores of 128^3 to 203 x 301 x 287 voxels, three shapes and both arithmetics.
-constexpr int kItemPlanes = 4;
-constexpr int kSegments[] = {64, 48, 40, 32, 24, 20, 16, 12, 10, 8, 6};
-
-// Expected time of the volumes' work items for rows x slices tiles (in planes of
-// one tile), and the segment length that gives it (`segment` > 0: that one).  A
-// block runs one item and `slots` blocks run at a time, so a volume of few tiles
-// leaves multiprocessors idle, or its last wave nearly empty, with long segments,
-// and pays kItemPlanes too often with short ones: 128^3 (radius 60, fast, 8 x
-// 128 tiles) takes 171 us per iteration with segments of 64 columns (30 items), 52
-// with 10 and 57 with 4.  The items go to the first free slot in order, as the
-// hardware hands out blocks; with at least kManyWaves items per slot their mean decides.
-constexpr int kManyWaves = 12;
-double march_time(const std::vector<MarchVolume> &vols, int rows, int slices, int slots, int segment, int *best)
-{
-    struct Run {
-        int len, tiles;
-    };
-    std::vector<Run> runs;
-    for (const MarchVolume &v : vols) {
-        const auto [lo, hi] = row_range(*v.map, v.c_begin, v.c_end);
-        const int tiles = (v.ns + slices - 1) / slices;
-        for (int r0 = lo; r0 < hi; r0 += rows)
-            for (const ColumnRun &r : tile_runs(*v.map, r0, rows, v.c_begin, v.c_end))
-                runs.push_back({r.second - r.first, tiles});
-    }
-    double best_time = -1.0;
-    std::vector<int> ends, lens;
-    for (int seg : kSegments) {
-        if (segment > 0) seg = segment;
-        int64_t items = 0, planes = 0;
-        int longest = 0;
-        for (const Run &r : runs) {
-            const int n = (r.len + seg - 1) / seg;
-            items += (int64_t)n * r.tiles;
-            planes += (int64_t)(r.len + n * kItemPlanes) * r.tiles;
-            longest = std::max(longest, (r.len + seg - 1) / seg);
-        }
-        double time = (double)planes / slots;
-        if (items < (int64_t)kManyWaves * slots && (best_time < 0.0 || time < best_time)) {
-            lens.clear();
-            for (int k = 0; k < longest; ++k)
-                for (const Run &r : runs)
-                    if (k * seg < r.len) lens.insert(lens.end(), (size_t)r.tiles, std::min(seg, r.len - k * seg));
-            ends.assign((size_t)slots, 0);  // a heap, the first free slot on top
-            for (int len : lens) {
-                std::pop_heap(ends.begin(), ends.end(), std::greater<int>());
-                ends.back() += len + kItemPlanes;
-                std::push_heap(ends.begin(), ends.end(), std::greater<int>());
-            }
-            time = (double)*std::max_element(ends.begin(), ends.end());
-        }
-        if (best_time < 0.0 || time < best_time) {
-            best_time = time;
-            *best = seg;
-        }
-        // many items with the longest segments: shorter ones only add planes
-        if (segment > 0 || (seg == kSegments[0] && items >= (int64_t)kManyWaves * slots)) break;
-    }
-    return best_time;
-}
-
 // Blocks per multiprocessor of each compiled shape.
 template <int K, typename ST, size_t... I>
 std::array<int, sizeof...(I)> shape_blocks(std::index_sequence<I...>)
@@ -706,6 +604,8 @@ int choose_tile(const potts_options &o, const std::vector<MarchVolume> &vols, in
     const bool named = o.tile_rows > 0 || o.tile_slices > 0 || o.tile_vpt > 0;
     const auto blocks = shape_blocks<K, ST>(std::make_index_sequence<(size_t)TS::n>());
     double best = -1.0;
+    std::vector<MarchRun> runs;  // of the tile height `height`
+    int height = 0;
     for (int i = 0; i < (named ? TS::named : TS::n); ++i) {
         if (named && !((o.tile_rows <= 0 || o.tile_rows == TS::r[i]) && (o.tile_slices <= 0 || o.tile_slices == TS::t[i]) &&
                        (o.tile_vpt <= 0 || o.tile_vpt == TS::v[i])))
@@ -714,7 +614,11 @@ int choose_tile(const potts_options &o, const std::vector<MarchVolume> &vols, in
         const int weight = o.arith == POTTS_ARITH_FAST ? TS::fast[i] : TS::exact[i];
         // b blocks on a multiprocessor share its rate
         const int b = blocks[(size_t)i];
-        const double time = march_time(vols, TS::r[i], TS::t[i], b * std::max(n_sm, 1), o.segment_cols, &segment) *
+        if (height != TS::r[i]) {
+            runs = march_runs(vols, TS::r[i]);
+            height = TS::r[i];
+        }
+        const double time = march_time(runs, TS::t[i], b * std::max(n_sm, 1), o.segment_cols, &segment) *
                             (weight * TS::r[i] * TS::t[i] * b);
         if (best < 0.0 || time < best) {
             best = time;
@@ -750,17 +654,19 @@ std::vector<int4> work_items(const potts_mapping &m, int ns, const TileChoice &t
     // the columns [c_begin, c_end) (default: all active columns)
     const int cb0 = c_begin < 0 ? (int)m.col_begin : c_begin;
     const int ce0 = c_end < 0 ? (int)m.col_end : c_end;
-    const auto [row_lo, row_hi] = row_range(m, cb0, ce0);
+    const std::vector<RowRange> cols = column_rows(m, cb0, ce0);
+    const RowRange all = row_range(cols);
     struct Item {
         int ca, r0, n0, cb;
     };
     std::vector<Item> items;
     const int tiles = (ns + tc.slices - 1) / tc.slices;
-    for (int r0 = row_lo; r0 < row_hi; r0 += tc.rows)
-        for (const ColumnRun &run : tile_runs(m, r0, tc.rows, cb0, ce0))
-            for (int ca = run.first; ca < run.second; ca += tc.segment)
+    for (int r0 = all.first; r0 < all.second; r0 += tc.rows)
+        tile_runs(cols, r0, tc.rows, [&](int first, int second) {
+            for (int ca = cb0 + first; ca < cb0 + second; ca += tc.segment)
                 for (int t = 0; t < tiles; ++t)
-                    items.push_back({ca, r0, t * tc.slices, std::min(run.second, ca + tc.segment)});
+                    items.push_back({ca, r0, t * tc.slices, std::min(cb0 + second, ca + tc.segment)});
+        });
     std::sort(items.begin(), items.end(), [](const Item &a, const Item &b) {
         if (a.ca != b.ca) return a.ca < b.ca;
         if (a.r0 != b.r0) return a.r0 < b.r0;
@@ -1324,8 +1230,8 @@ int tv_tiled_setup(potts_context *ctx, const Geometry &g, const float *xi_a, con
     using T = potts::TvTile;
     const potts_mapping &m = ctx->mapping.m;
     int segment = 64;
-    march_time({{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, T::TR, T::TN, potts::kTvBlocks * std::max(ctx->n_sm, 1), 0,
-               &segment);
+    march_time(march_runs({{&m, g.ns, (int)m.col_begin, (int)m.col_end}}, T::TR), T::TN,
+               potts::kTvBlocks * std::max(ctx->n_sm, 1), 0, &segment);
     POTTS_TRY(plan_tiles(ctx, g.ns, TileChoice{T::TR, T::TN, 4, segment}));
     POTTS_CUDA(cudaFuncSetAttribute(potts::tv_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     T::SMEM_BYTES));
