@@ -2,15 +2,21 @@
 // slices x slices per thread; W = 4 for FP32, 2 for the 16-bit formats), each in
 // the exact and the fast arithmetic (fused_*.cu).  Options can name the first
 // `named` entries.  exact / fast: time per voxel of a full tile relative to the
-// best shape's (per cent), measured on a 448 x 448 x 256 core of radius 215 over
-// the iterations 2 to 24; choose_tile weighs a volume's ragged tiles with them.
-// Best shapes per iteration: K = 3 FP32 exact 0.844 ms (8 x 128 x 4; 16 x 64 x 2 0.871,
-// but 15 % faster where few voxels run the projection loop, 0.89 against 1.05 ms
-// at 4 % of them on 512 x 512 x 256: its weight is below), fast 0.593, bf16 0.882
-// and 0.605; K = 4 1.36 and 0.978; K = 5 2.09 and 1.24; K = 2 (512 x 512 x 256,
-// iterations 2 to 40, 8 x 64 x 4 with two blocks per multiprocessor) 0.589 and
-// 0.452.  A K = 3 tile of 8 x 64 x 4 with two blocks measured 0.840 against 0.806
-// ms fast and 1.33 against 1.17 exact there.
+// best shape's (per cent); choose_tile weighs a volume's ragged tiles with them.
+// Which shape is best depends on the share of voxels in the projection loop.  K = 3 FP32
+// exact: the weights that give the least time over 26 cores of 0.6 to 60 million voxels
+// with grains of 16, 48 and 160 voxels (50 iterations): 3.5 % above the best shape on
+// average.  {100, 109, 106, 104}, from small grains on one core, took 8 x 64 x 2 for
+// 200^3 to 440^3 cores: 6 % above, and 1.11 against 0.91 ms on a smooth 440^3 field.  K = 2 and
+// K = 4 FP32 and K = 3 fast and 16-bit: measured on a 448 x 448 x 256 core of radius 215 with
+// small grains (16-bit K = 2: FP32's); on average over the 26 cores at most 5 % above the
+// best shape.  K = 5 and K = 6: means over cubic grains of 200, 56 and 14 voxels on a 512 x
+// 512 x 256 core.
+// Best shapes per iteration on the 14-voxel grains there, exact and fast: K = 2 0.546 and
+// 0.428 ms, K = 3 1.334 (8 x 128 x 4; 16 x 64 x 2 1.387) and 0.880, 16-bit 1.452 and 0.933, K = 4
+// 2.99 and 1.66, K = 5 6.22 and 2.91, K = 6 24.6 and 9.2 (4 x 64 x 4; 16-bit with 8 x 64 x 2:
+// 11.7 and 4.7).  A K = 3 tile of 8 x 64 x 4 with two blocks per multiprocessor measured
+// 0.840 against 0.806 ms fast and 1.33 against 1.17 exact on 512 x 512 x 256.
 #pragma once
 
 namespace potts {
@@ -18,13 +24,14 @@ namespace potts {
 template <int K, int W>
 struct TileShapes;
 template <int W> struct TileShapes<2, W> { static constexpr int n = 2, named = 2; static constexpr int r[n] = {8, 8}, t[n] = {128, 64}, v[n] = {2, 4}, exact[n] = {104, 100}, fast[n] = {108, 100}; };
-template <> struct TileShapes<3, 4> { static constexpr int n = 4, named = 4; static constexpr int r[n] = {16, 8, 8, 8}, t[n] = {64, 128, 64, 128}, v[n] = {2, 2, 2, 4}, exact[n] = {100, 109, 106, 104}, fast[n] = {107, 113, 123, 100}; };
+template <> struct TileShapes<3, 4> { static constexpr int n = 4, named = 4; static constexpr int r[n] = {16, 8, 8, 8}, t[n] = {64, 128, 64, 128}, v[n] = {2, 2, 2, 4}, exact[n] = {104, 102, 121, 100}, fast[n] = {107, 113, 123, 100}; };
 template <> struct TileShapes<3, 2> { static constexpr int n = 3, named = 2; static constexpr int r[n] = {16, 8, 8}, t[n] = {64, 128, 128}, v[n] = {2, 2, 4}, exact[n] = {100, 112, 108}, fast[n] = {109, 120, 100}; };
 template <> struct TileShapes<4, 4> { static constexpr int n = 3, named = 3; static constexpr int r[n] = {8, 8, 4}, t[n] = {64, 64, 128}, v[n] = {2, 4, 4}, exact[n] = {100, 170, 162}, fast[n] = {100, 116, 110}; };
 template <> struct TileShapes<4, 2> { static constexpr int n = 1, named = 1; static constexpr int r[n] = {8}, t[n] = {64}, v[n] = {2}, exact[n] = {100}, fast[n] = {100}; };
-template <int W> struct TileShapes<5, W> { static constexpr int n = 2, named = 2; static constexpr int r[n] = {4, 8}, t[n] = {64, 64}, v[n] = {4, 2}, exact[n] = {261, 100}, fast[n] = {201, 100}; };
+template <> struct TileShapes<5, 4> { static constexpr int n = 2, named = 2; static constexpr int r[n] = {4, 8}, t[n] = {64, 64}, v[n] = {4, 2}, exact[n] = {214, 100}, fast[n] = {162, 100}; };
+template <> struct TileShapes<5, 2> { static constexpr int n = 2, named = 2; static constexpr int r[n] = {4, 8}, t[n] = {64, 64}, v[n] = {4, 2}, exact[n] = {172, 100}, fast[n] = {142, 100}; };
 template <> struct TileShapes<6, 4> { static constexpr int n = 1, named = 1; static constexpr int r[n] = {4}, t[n] = {64}, v[n] = {4}, exact[n] = {100}, fast[n] = {100}; };
-template <> struct TileShapes<6, 2> { static constexpr int n = 2, named = 2; static constexpr int r[n] = {4, 8}, t[n] = {64, 64}, v[n] = {4, 2}, exact[n] = {250, 100}, fast[n] = {200, 100}; };
+template <> struct TileShapes<6, 2> { static constexpr int n = 2, named = 2; static constexpr int r[n] = {4, 8}, t[n] = {64, 64}, v[n] = {4, 2}, exact[n] = {179, 100}, fast[n] = {167, 100}; };
 
 template <int K, typename ST>
 using ShapesOf = TileShapes<K, (int)sizeof(ST) == 4 ? 4 : 2>;
