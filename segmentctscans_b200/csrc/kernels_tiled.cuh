@@ -86,21 +86,11 @@ struct TileShape {
     static constexpr int NV = NT + 4;                   // u and Vbar (FP32): slices n0 .. n0+NT+3
     static constexpr int MAIN = R * Q;
     static constexpr int MAIN_WARPS = MAIN / 32;
-    // the high halo row, then (its own warp when POTTS_NHALO_WARP) the slice n0+NT
-#ifdef POTTS_NHALO_WARP
-    static constexpr int NHALO_OWN = 1;
-#else
-    static constexpr int NHALO_OWN = 0;
-#endif
-    static constexpr int HALO_WARPS = (Q + 31) / 32 + NHALO_OWN;
+    static constexpr int HALO_WARPS = (Q + 31) / 32;  // the high halo row and the slice n0+NT
     static constexpr int PRODUCER_WARP = MAIN_WARPS + HALO_WARPS;
     // Dykstra warps run the projection loop of queued voxels: warp w serves the
     // queues of the row warps w, w + NW, ...
-#ifdef POTTS_DYKSTRA_WARPS
-    static constexpr int NW = MAIN_WARPS >= 2 * POTTS_DYKSTRA_WARPS ? POTTS_DYKSTRA_WARPS : (MAIN_WARPS >= 2 ? MAIN_WARPS / 2 : 1);
-#else
     static constexpr int NW = MAIN_WARPS >= 12 ? (HALO_WARPS > 1 ? 5 : 6) : (MAIN_WARPS >= 2 ? MAIN_WARPS / 2 : 1);
-#endif
     static constexpr int QPW = (MAIN_WARPS + NW - 1) / NW;  // queues per Dykstra warp
     static constexpr int DYKSTRA_WARP = PRODUCER_WARP + 1;  // the first one
     static constexpr int THREADS = MAIN + 32 * HALO_WARPS + 32 + 32 * NW;
@@ -900,9 +890,7 @@ __device__ __forceinline__ void tiled_item(const TiledSmem<K, R, NT, VPT, ST> &s
             const int rr = is_main ? tid / S::Q : R;
             const int q = is_main ? tid % S::Q : hq;
             const bool chunk_a = is_main || hq < S::Q;
-            // lanes of the first halo warp, or of the last one when it has its own
-            const int hn = S::NHALO_OWN ? hq - 32 * (S::HALO_WARPS - 1) : hq;
-            const bool nhalo = !is_main && hn >= 0 && hn <= R;
+            const bool nhalo = !is_main && hq >= 0 && hq <= R;  // (without hq >= 0 the 80-register tiles spill)
             bool ok = true;
             // ring slots of positions p-1, p, p+1 and the barrier parities of p-1, p
             int s_prev = S::D - 1, s_cur = 0, s_next = 1;
@@ -915,7 +903,7 @@ __device__ __forceinline__ void tiled_item(const TiledSmem<K, R, NT, VPT, ST> &s
                     if (chunk_a)
                         stage_a_chunk<K, R, NT, VPT, ST, FAST>(sm, tp, pp, p, s_cur, s_prev, r0, rr, n0, q,
                                                          is_main && ca - 1 + p < cb, Vout, dqmax);
-                    if (nhalo) stage_a_nhalo<K, R, NT, VPT, ST, FAST>(sm, tp, pp, p, s_cur, s_prev, r0, hn, n0);
+                    if (nhalo) stage_a_nhalo<K, R, NT, VPT, ST, FAST>(sm, tp, pp, p, s_cur, s_prev, r0, hq, n0);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sm.ready(s_cur));
