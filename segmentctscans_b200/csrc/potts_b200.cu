@@ -677,12 +677,23 @@ std::vector<int4> work_items(const potts_mapping &m, int ns, const TileChoice &t
     return work;
 }
 
+// Tables are not copied under stream capture: the copy would become a node of the graph and read the table's
+// host memory, which ends with the call, at every replay.  The call is to run once before it is captured.
+int may_upload(potts_context *ctx)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    POTTS_CUDA(cudaStreamIsCapturing(ctx->stream, &st));
+    if (st == cudaStreamCaptureStatusNone) return POTTS_OK;
+    return fail(POTTS_ECUDA, "the call's work list is not on the device, which a stream capture does not allow");
+}
+
 // Host tables to device memory in the order of the context's stream: a table that earlier calls' kernels may
 // still be reading is overwritten behind them.  (cudaMemcpy orders itself by the default stream only; the
 // pageable source is staged before this returns.)
 template <typename T>
 int upload_table(potts_context *ctx, void *dst, const std::vector<T> &src, size_t n)
 {
+    POTTS_TRY(may_upload(ctx));
     if (n > 0) POTTS_CUDA(cudaMemcpyAsync(dst, src.data(), sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream));
     return POTTS_OK;
 }
@@ -692,6 +703,7 @@ int plan_tiles(potts_context *ctx, int ns, const TileChoice &tc)
 {
     const MappingCopy &mc = ctx->mapping;
     if (!ctx->cols_valid) {
+        POTTS_TRY(may_upload(ctx));
         const std::vector<int4> cols = column_table(mc.m);
         POTTS_TRY(ensure(ctx, ctx->cols, sizeof(int4) * cols.size()));
         POTTS_TRY(upload_table(ctx, ctx->cols.p, cols, cols.size()));
@@ -699,6 +711,8 @@ int plan_tiles(potts_context *ctx, int ns, const TileChoice &tc)
     }
     const int key[5] = {ns, tc.rows, tc.slices, tc.segment, (int)mc.n_lines};
     if (std::equal(key, key + 5, ctx->work_key)) return POTTS_OK;
+    POTTS_TRY(may_upload(ctx));
+    ctx->work_key[0] = -1;  // the list is no plan's until the new one is there
     const std::vector<int4> work = work_items(mc.m, ns, tc);
     POTTS_TRY(ensure(ctx, ctx->work, sizeof(int4) * std::max<size_t>(work.size(), 1)));
     POTTS_TRY(upload_table(ctx, ctx->work.p, work, work.size()));
