@@ -106,12 +106,14 @@ typedef struct potts_options {
     int tile_rows;    /* fused form: rows per tile (0 = chosen by K, arith and the volume's size) */
     int tile_slices;  /* fused form: slices (n) per tile (0 = chosen likewise) */
     int segment_cols; /* fused form: columns one tile marches over (0 = chosen by the volume's size, at most 64) */
-    int tile_vpt;     /* fused form: consecutive slices per thread, 2 or 4 (0 = chosen likewise) */
+    int tile_vpt;     /* fused form: consecutive slices per thread, 2 or 4 (0 = chosen likewise; the choice
+                         also has shapes that cannot be named: 8 x 128 x 4 of K = 3 with 16-bit state) */
     int prefetch;     /* fused form: planes the load ring prefetches into L2 ahead of its loads
                          (0 = default: none, < 0 = none, at most 16) */
-    int autotune;     /* batches: 1 = time every compiled tile shape and segment length, each as one
-                         launch per iteration and as the persistent launch, on the batch and keep the
-                         fastest (used when no tile option is set); 0 = default tile and launch form */
+    int autotune;     /* batches: 1 = time every compiled tile shape with segments of 16, 32 and 64
+                         columns, each as one launch per iteration and as the persistent launch, on the
+                         batch and keep the fastest (used when no tile option is set); 0 = tile and segment
+                         chosen by the volumes' sizes, out of more lengths, one launch per iteration */
     int arith;        /* enum potts_arith (default EXACT) */
     int stall_plane;  /* testing the bounded waits: > 0 makes the fused kernel's first work item skip
                          the loads of that plane of its column march, so every wait for it gives up
@@ -264,8 +266,9 @@ int potts_energies_static(const potts_mapping *map, const float *d_u, int K, con
  * outputs again (u may change between runs; the pointers may not).  The fused
  * form only (opts->variant is ignored), no slabs (the state of all volumes must
  * fit in device memory, else POTTS_ENOMEM), gap_every is ignored.  Tile shape:
- * the options', or with opts->autotune = 1 the fastest compiled shape and
- * segment length measured on the batch (results do not depend on it).
+ * the options', or chosen by the volumes' sizes, or with opts->autotune = 1 the
+ * fastest compiled shape and segment length (of 16, 32 and 64 columns) measured on
+ * the batch (results do not depend on it).
  * ------------------------------------------------------------------------- */
 typedef struct potts_batch potts_batch;
 
